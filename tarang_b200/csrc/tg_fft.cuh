@@ -105,59 +105,6 @@ __global__ void __launch_bounds__(256) k_axis_c2c(AxisArgs a, PtrSet ps) {
 }
 
 // ------------------------------------------------------------------------------------------
-// strided-axis direct DFT for any L (used for lengths that are not a power of two)
-// block = 256 threads, 8 columns, tile [L][8] in shared memory
-// ------------------------------------------------------------------------------------------
-template <typename Ri, typename Ro, typename Rw, int DIR>
-__global__ void __launch_bounds__(256) k_axis_dft(AxisArgs a, PtrSet ps, int L) {
-  constexpr int W = 8;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cx<Rw>* tw = reinterpret_cast<cx<Rw>*>(smem_raw);
-  cx<Rw>* tile = tw + L;
-  const int tid = threadIdx.x;
-  const int f = blockIdx.z;
-  const cx<Ri>* src = reinterpret_cast<const cx<Ri>*>(ps.src[f]) + (long long)blockIdx.y * a.sb;
-  cx<Ro>* dst = reinterpret_cast<cx<Ro>*>(ps.dst[f]) + (long long)blockIdx.y * a.db;
-  const int comb = a.comb[f];
-  const cx<Ri>* src2 = comb ? reinterpret_cast<const cx<Ri>*>(ps.src2[f]) + (long long)blockIdx.y * a.sb : src;
-  const int c0 = blockIdx.x * W;
-  for (int i = tid; i < L; i += 256) {
-    cx<Rw> t = cvt<Rw>(a.tw[i]);
-    if (DIR > 0) t.y = -t.y;
-    tw[i] = t;
-  }
-  for (int i = tid; i < L * W; i += 256) {
-    const int n = i / W, w = i % W;
-    const int r = amap_row(a.in, n);
-    const int col = c0 + w;
-    cx<Rw> v = mkc<Rw>(0, 0);
-    if (col < a.ncols && r >= 0) {
-      const long long o = (long long)r * a.sr + col;
-      v = cvt<Rw>(src[o]);
-      if (comb > 0) v = v + cvt<Rw>(src2[o]);
-      else if (comb < 0) v = v - cvt<Rw>(src2[o]);
-    }
-    tile[i] = v;
-  }
-  __syncthreads();
-  const Rw sc = (Rw)a.scale;
-  for (int i = tid; i < L * W; i += 256) {
-    const int k = i / W, w = i % W;
-    const int r = amap_row(a.out, k);
-    const int col = c0 + w;
-    if (col >= a.ncols || r < 0) continue;
-    cx<Rw> acc = mkc<Rw>(0, 0);
-    int m = 0;
-    for (int n = 0; n < L; ++n) {
-      acc = acc + tile[n * W + w] * tw[m];
-      m += k;
-      if (m >= L) m -= L;
-    }
-    dst[(long long)r * a.dr + col] = cvt<Ro>(sc * acc);
-  }
-}
-
-// ------------------------------------------------------------------------------------------
 // SCFT x-pass: real-to-real transforms along axis 1 on complex columns (the real and imaginary
 // parts transform alike, as the reference's separate calls on real() and imag() do,
 // scft_tr.cc:249-259).  With t[j] = (cos, sin)(pi j / 2N), j in [0, 4N):

@@ -3,14 +3,16 @@
 // Power-of-two lengths 16..256 whose stored input and kept output rows fit one TMA box (<= 256
 // rows) run k_axis_tma: the block's column tile moves HBM -> shared memory and back as single
 // tiled bulk tensor copies, so the threads spend no instructions on addresses or row maps of
-// global memory.  Other lengths run the register-staged k_axis_c2c / k_axis_dft.  Both compute
-// the same butterflies in the same order (equal results up to how the compiler contracts
-// multiply-adds in each kernel).
+// global memory.  Power-of-two lengths beyond that run the register-staged k_axis_c2c, every
+// other length the mixed-radix k_axis_mixed.  k_axis_tma and k_axis_c2c compute the same
+// butterflies in the same order (equal results up to how the compiler contracts multiply-adds in
+// each kernel).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
 
 #include "tg_fft_launch.h"
+#include "tg_fft_mixed.cuh"
 #include "tg_fft_tc.cuh"
 #include "tg_tma.cuh"
 
@@ -227,14 +229,28 @@ cudaError_t run_axis_fast(const AxisLaunch& l, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// lengths that are no power of two (or beyond the register-staged kernels): the mixed-radix
+// Stockham pass.  Eight columns a tile while two tiles fit beside another block's, else four, two
+// or one.  Threads: what the stage of most butterflies has work for, at most kMixThreads.
 template <typename Ri, typename Ro, typename Rw, int DIR>
-cudaError_t run_axis_dft(const AxisLaunch& l, cudaStream_t s) {
-  const size_t smem = (size_t)(l.L + (size_t)l.L * 8) * sizeof(cx<Rw>);
-  auto kern = k_axis_dft<Ri, Ro, Rw, DIR>;
+cudaError_t run_axis_mixed(const AxisLaunch& l, cudaStream_t s) {
+  MixPlan p;
+  if (!mix_plan(l.L, p)) return cudaErrorInvalidValue;
+  auto bytes = [&](int w) { return (size_t)(l.L + ((size_t)l.L << (w + 1))) * sizeof(cx<Rw>); };
+  while (p.wsh > 0 && bytes(p.wsh) > 100 * 1024) --p.wsh;
+  const size_t smem = bytes(p.wsh);
+  if (smem > 227 * 1024) return cudaErrorInvalidValue;
+  int threads = 32;
+  for (int i = 0; i < p.ns; ++i) {
+    const int items = mix_reg_radix(p.r[i]) ? (l.L / p.r[i]) << p.wsh : l.L << p.wsh;
+    threads = std::max(threads, std::min(kMixThreads, (items + 31) / 32 * 32));
+  }
+  const int W = 1 << p.wsh;
+  auto kern = k_axis_mixed<Ri, Ro, Rw, DIR>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  dim3 grid((l.a.ncols + 7) / 8, l.nbatch, l.nfields);
-  kern<<<grid, 256, smem, s>>>(l.a, l.ps, l.L);
+  dim3 grid((l.a.ncols + W - 1) / W, l.nbatch, l.nfields);
+  kern<<<grid, threads, smem, s>>>(l.a, l.ps, p);
   return cudaGetLastError();
 }
 
@@ -252,7 +268,7 @@ cudaError_t run_axis_dir(const AxisLaunch& l, cudaStream_t s) {
     case 512: return run_axis_fast<Ri, Ro, Rw, 32, 16, DIR>(l, s);
     default:
       if (l.L < 1 || l.L > 2048) return cudaErrorInvalidValue;
-      return run_axis_dft<Ri, Ro, Rw, DIR>(l, s);
+      return run_axis_mixed<Ri, Ro, Rw, DIR>(l, s);
   }
 }
 
