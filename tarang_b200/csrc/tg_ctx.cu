@@ -704,7 +704,8 @@ int ctx_create_batch(const tg_config* cfg, int B, tg_ctx** out, int slab_W, int 
       h[j].y = (double)sinl(ang);
     }
     if ((rc = dalloc(c, (void**)&c->trigx, sizeof(cx<double>) * h.size()))) return fail(rc);
-    e = cudaMemcpy(c->trigx, h.data(), sizeof(cx<double>) * h.size(), cudaMemcpyHostToDevice);
+    // on the context's stream, behind the allocation's clearing (as the other tables)
+    e = cudaMemcpyAsync(c->trigx, h.data(), sizeof(cx<double>) * h.size(), cudaMemcpyHostToDevice, c->st);
     if (e != cudaSuccess) return fail(cuda_err(c, e, "trig table"));
     // the x-pass of the pipeline as matrices [stored input row][output row] (the coefficients
     // of k_axis_r2r): inverse kinds 2, 3 map the nkx stored slots m to all N1 points,
@@ -729,7 +730,7 @@ int ctx_create_batch(const tg_config* cfg, int B, tg_ctx** out, int slab_W, int 
           m[(size_t)rr * nout + ko] = t;
         }
       if ((rc = dalloc(c, (void**)&c->xmat[kind], sizeof(double) * m.size()))) return fail(rc);
-      e = cudaMemcpy(c->xmat[kind], m.data(), sizeof(double) * m.size(), cudaMemcpyHostToDevice);
+      e = cudaMemcpyAsync(c->xmat[kind], m.data(), sizeof(double) * m.size(), cudaMemcpyHostToDevice, c->st);
       if (e != cudaSuccess) return fail(cuda_err(c, e, "x-pass matrices"));
       c->xmat_rows[kind] = nout;
       c->xmat_cols[kind] = nin;
@@ -743,7 +744,7 @@ int ctx_create_batch(const tg_config* cfg, int B, tg_ctx** out, int slab_W, int 
     std::vector<cx<double>> t(kZoctTableLen);
     zoct_table(N3 / 2, t.data());
     if ((rc = dalloc(c, (void**)&c->zoct, sizeof(cx<double>) * t.size()))) return fail(rc);
-    e = cudaMemcpy(c->zoct, t.data(), sizeof(cx<double>) * t.size(), cudaMemcpyHostToDevice);
+    e = cudaMemcpyAsync(c->zoct, t.data(), sizeof(cx<double>) * t.size(), cudaMemcpyHostToDevice, c->st);
     if (e != cudaSuccess) return fail(cuda_err(c, e, "z-pass table"));
   }
   // a batch of B same-shape requests stores request r of every field at offset r * S
