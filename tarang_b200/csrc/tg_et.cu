@@ -224,15 +224,6 @@ __global__ void __launch_bounds__(TPB) k_et_contract(ContractArgs a) {
   }
 }
 
-// hist[i] = the blocks' sums of bin i in block order (one thread per bin)
-__global__ void k_et_reduce(const double* __restrict__ part, int nblocks, int nbins, double* hist) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nbins) return;
-  double t = 0;
-  for (int b = 0; b < nblocks; ++b) t += part[(size_t)b * nbins + i];
-  hist[i] = t;
-}
-
 struct KindSpec {
   int H, F;      // field groups: 0 = U (state 0..2), 1 = B (state 3..5)
   int R;         // receiver group
@@ -322,9 +313,8 @@ int et_tables_ptr(tg_ctx* c, const cx<double>* const* Hp, const cx<double>* cons
       ProfScope pr(c, "et_contract", 0.0);
       if (c->tprec == F64) k_et_contract<double><<<nblk, TPB, 0, c->st>>>(a);
       else k_et_contract<float><<<nblk, TPB, 0, c->st>>>(a);
-      k_et_reduce<<<(nrec * nb + 127) / 128, 128, 0, c->st>>>(a.part, nblk, nrec * nb, a.hist);
+      e = launch_bins_accumulate(a.part, nblk, nrec * nb, a.hist, nrec * nb, nullptr, c->st);  // hist is zeroed
     }
-    e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_err(c, e, "et contract");
   }
   std::vector<double> h(need);

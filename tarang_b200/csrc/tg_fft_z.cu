@@ -178,12 +178,14 @@ int oct_phys(const ProdPairs& pp) {
   static const signed char F_A[6] = {0, 1, 2, 0, 1, 2}, F_B[6] = {0, 1, 2, 1, 2, 0};
   static const signed char M_A[9] = {0, 1, 2, 0, 3, 1, 4, 2, 5}, M_B[9] = {3, 4, 5, 4, 1, 5, 2, 3, 0};
   static const signed char S_A[9] = {0, 1, 2, 0, 1, 2, 0, 1, 2}, S_B[9] = {0, 1, 2, 1, 2, 0, 3, 3, 3};
+  static const signed char E_A[9] = {3, 3, 3, 4, 4, 4, 5, 5, 5}, E_B[9] = {0, 1, 2, 0, 1, 2, 0, 1, 2};
   const signed char *A, *B;
   int ph;
   if (NIN == 3 && NPROD == 6) {
     A = F_A, B = F_B, ph = 0;
   } else if (NIN == 6 && NPROD == 9) {
-    A = M_A, B = M_B, ph = 1;
+    if (pp.a[0] == 0) A = M_A, B = M_B, ph = 1;
+    else A = E_A, B = E_B, ph = 3;
   } else if (NIN == 4 && NPROD == 9) {
     A = S_A, B = S_B, ph = 2;
   } else {
@@ -219,6 +221,7 @@ cudaError_t run_zprod_oct_any(const ZProdLaunch& l, int ph, cudaStream_t s) {
   const bool prune = l.a.nin <= 96 && l.a.nout <= 96;
   if (ph == 0) return prune ? run_zprod_oct<Ri, Ro, Rw, 0, true>(l, s) : run_zprod_oct<Ri, Ro, Rw, 0, false>(l, s);
   if (ph == 1) return prune ? run_zprod_oct<Ri, Ro, Rw, 1, true>(l, s) : run_zprod_oct<Ri, Ro, Rw, 1, false>(l, s);
+  if (ph == 3) return prune ? run_zprod_oct<Ri, Ro, Rw, 3, true>(l, s) : run_zprod_oct<Ri, Ro, Rw, 3, false>(l, s);
   return prune ? run_zprod_oct<Ri, Ro, Rw, 2, true>(l, s) : run_zprod_oct<Ri, Ro, Rw, 2, false>(l, s);
 }
 
@@ -247,6 +250,7 @@ cudaError_t run_zprod_oct64_any(const ZProdLaunch& l, int ph, cudaStream_t s) {
   const bool prune = l.a.nin <= 48 && l.a.nout <= 48;
   if (ph == 0) return prune ? run_zprod_oct64<Ri, Ro, Rw, 0, true>(l, s) : run_zprod_oct64<Ri, Ro, Rw, 0, false>(l, s);
   if (ph == 1) return prune ? run_zprod_oct64<Ri, Ro, Rw, 1, true>(l, s) : run_zprod_oct64<Ri, Ro, Rw, 1, false>(l, s);
+  if (ph == 3) return prune ? run_zprod_oct64<Ri, Ro, Rw, 3, true>(l, s) : run_zprod_oct64<Ri, Ro, Rw, 3, false>(l, s);
   return prune ? run_zprod_oct64<Ri, Ro, Rw, 2, true>(l, s) : run_zprod_oct64<Ri, Ro, Rw, 2, false>(l, s);
 }
 

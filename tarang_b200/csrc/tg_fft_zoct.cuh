@@ -66,9 +66,10 @@ __device__ __forceinline__ cx<R> cmul_conjb(cx<R> a, cx<R> b) {  // a conj(b)
 //   1 MHD     inputs z+1..3 (parked), z-1..3 (registers); PA = {0,1,2,0,3,1,4,2,5},
 //             PB = {3,4,5,4,1,5,2,3,0}: each product pairs one z+ with one z-
 //   2 scalar  inputs u1 u2 u3 (parked), theta (registers); products as fluid, then u_i theta
+//   3 energy transfer  inputs H1..3 (parked), G1..3 (registers); product 3 i + j = G_i H_j (tg_et.cu)
 template <int PHYS>
 struct OctLayout {
-  static constexpr int nin = PHYS == 1 ? 6 : (PHYS == 2 ? 4 : 3);
+  static constexpr int nin = (PHYS == 1 || PHYS == 3) ? 6 : (PHYS == 2 ? 4 : 3);
   static constexpr int npark = 3;
 };
 // MHD: the three products of register input z-(3 + i), j-th of them: product index and the
@@ -477,7 +478,7 @@ __global__ void __launch_bounds__(128, OctOcc<Rw, PHYS>::v) k_z_prod_oct(ZArgs a
         L.template forward<Ro, PRUNE>(v, Y, a.nout, a.nfill);
       }
     }
-    if constexpr (PHYS == 1 || PHYS == 2) {
+    if constexpr (PHYS != 0) {
       // register inputs, each multiplied with the three parked inputs
 #pragma unroll 1
       for (int c = 3; c < Lay::nin; ++c) {
@@ -486,8 +487,9 @@ __global__ void __launch_bounds__(128, OctOcc<Rw, PHYS>::v) k_z_prod_oct(ZArgs a
         L.template inverse<Ri, PRUNE>(X, a.nin, w);
 #pragma unroll 1
         for (int j = 0; j < 3; ++j) {
-          // PHYS 2: product 6 + j = u_j theta; PHYS 1: the three products of z-(c) in order
-          int q = 6 + j, pa = j;
+          // PHYS 2: product 6 + j = u_j theta; PHYS 3: product 3 i + j = H_j G_i; PHYS 1: the three
+          // products of z-(c) in order
+          int q = (PHYS == 3 ? 3 * (c - 3) : 6) + j, pa = j;
           if constexpr (PHYS == 1) {
             const int sh = 4 * (3 * (c - 3) + j);
             q = (int)((kOctMhdQ >> sh) & 15);

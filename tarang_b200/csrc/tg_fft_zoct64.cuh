@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(128, Oct64Occ<Rw, PHYS>::v) k_z_prod_oct64(ZAr
         L.template forward<Ro, PRUNE>(v, Y, a.nout, a.nfill);
       }
     }
-    if constexpr (PHYS == 1 || PHYS == 2) {
+    if constexpr (PHYS != 0) {
       // register inputs, each multiplied with the three parked inputs
 #pragma unroll 1
       for (int c = 3; c < Lay::nin; ++c) {
@@ -286,8 +286,9 @@ __global__ void __launch_bounds__(128, Oct64Occ<Rw, PHYS>::v) k_z_prod_oct64(ZAr
         L.template inverse<Ri, PRUNE>(X, a.nin, w);
 #pragma unroll 1
         for (int j = 0; j < 3; ++j) {
-          // PHYS 2: product 6 + j = u_j theta; PHYS 1: the three products of z-(c) in order
-          int q = 6 + j, pa = j;
+          // PHYS 2: product 6 + j = u_j theta; PHYS 3: product 3 i + j = H_j G_i; PHYS 1: the three
+          // products of z-(c) in order
+          int q = (PHYS == 3 ? 3 * (c - 3) : 6) + j, pa = j;
           if constexpr (PHYS == 1) {
             const int sh = 4 * (3 * (c - 3) + j);
             q = (int)((kOctMhdQ >> sh) & 15);
