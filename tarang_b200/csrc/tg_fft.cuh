@@ -4,8 +4,8 @@
 //   x-pass : batched c2c along axis 1 (row stride N2*(N3/2+1)),   kernel k_axis_c2c
 //   y-pass : batched c2c along axis 2 (row stride N3/2+1),         kernel k_axis_c2c
 //   z-pass : c2r / r2c along the contiguous axis 3 via a length-N3/2 complex FFT,
-//            kernels k_z_c2r / k_z_r2c, or k_z_prod which fuses the inverse of several
-//            fields, their pointwise real-space products and the forward of every product.
+//            kernels k_z_c2r / k_z_r2c, or the k_z_prod_* kernels which fuse the inverse of
+//            several fields, their pointwise real-space products and the forward of every product.
 // Each pass reads and writes HBM once.  Inside a block the FFT of length L = R1*R2 is a
 // two-step (four-step) FFT: a radix-R1 register DFT per thread, a twiddle, one transpose
 // through shared memory, and a radix-R2 register DFT.  Axis maps (AxisMap) let a pass read
@@ -505,101 +505,15 @@ __global__ void __launch_bounds__(128) k_z_r2c_dft(ZArgs a, PtrSet ps, int M) {
 // ------------------------------------------------------------------------------------------
 // Fused z-pass of the nonlinear term: inverse (c2r) of NIN fields, NPROD pointwise real-space
 // products (pairs of inputs), forward (r2c) of every product with scale 1/(N1 N2 N3).
-// Between the inverse and the forward FFT each thread keeps the same positions
-// m = k1 + R1 k2, which are exactly the inputs of the forward FFT's first step with the radix
-// roles swapped, so the products are formed without another exchange.
+// The forward FFT runs the inverse's steps backwards, so a thread's real-space positions are the
+// ones it needs again and the products are formed without another exchange.
 // ------------------------------------------------------------------------------------------
 struct ProdPairs {
   signed char a[12], b[12];
 };
 
-template <typename Ri, typename Ro, typename Rw, int R1, int R2, int NIN, int NPROD>
-__global__ void __launch_bounds__(256 / ((R1 * R2 >= 128) ? 2 : 1))
-    k_z_prod(ZArgs a, PtrSet ps, ProdPairs pp) {
-  constexpr int M = R1 * R2;
-  constexpr int T = R1;
-  constexpr int ROWS = (256 / ((M >= 128) ? 2 : 1)) / T;
-  constexpr int EXA = R2 + 1;   // inverse exchange pitch
-  constexpr int EXB = R1 + 1;   // forward exchange pitch
-  constexpr int EXS = (R1 * EXA > R2 * EXB) ? R1 * EXA : R2 * EXB;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cx<Rw>* twM = reinterpret_cast<cx<Rw>*>(smem_raw);
-  cx<Rw>* twN = twM + M;
-  cx<Rw>* ex = twN + 2 * M;
-  cx<Rw>* zb = ex + ROWS * EXS;
-  cx<Rw>* rs = zb + ROWS * M;  // [NIN][ROWS][M]
-  const int tid = threadIdx.x;
-  for (int i = tid; i < M; i += blockDim.x) twM[i] = cvt<Rw>(a.twM[i]);
-  for (int i = tid; i < 2 * M; i += blockDim.x) twN[i] = cvt<Rw>(a.twN[i]);
-  const int rl = tid / T, t = tid % T;
-  const long long row = (long long)blockIdx.x * ROWS + rl;
-  const bool ok = row < a.nrows;
-  cx<Rw>* exr = ex + rl * EXS;
-  cx<Rw>* zr = zb + rl * M;
-  __syncthreads();
-#pragma unroll 1
-  for (int c = 0; c < NIN; ++c) {
-    const cx<Ri>* src = reinterpret_cast<const cx<Ri>*>(ps.src[c]) + row * a.ss;
-    if (t < R2) {
-      cx<Rw> v[R1];
-#pragma unroll
-      for (int n1 = 0; n1 < R1; ++n1)
-        v[n1] = ok ? c2r_pre<Rw>(src, R2 * n1 + t, M, a.nin, twN) : mkc<Rw>(0, 0);
-      DFT<R1, +1, Rw>::run(v);
-#pragma unroll
-      for (int k1 = 0; k1 < R1; ++k1) {
-        cx<Rw> w = twM[(t * k1) & (M - 1)];
-        w.y = -w.y;
-        exr[k1 * EXA + t] = v[k1] * w;
-      }
-    }
-    __syncthreads();
-    {
-      cx<Rw> v[R2];
-#pragma unroll
-      for (int n2 = 0; n2 < R2; ++n2) v[n2] = exr[t * EXA + n2];
-      DFT<R2, +1, Rw>::run(v);
-      cx<Rw>* rsr = rs + ((long long)c * ROWS + rl) * M;
-#pragma unroll
-      for (int k2 = 0; k2 < R2; ++k2) rsr[t + R1 * k2] = v[k2];
-    }
-    __syncthreads();
-  }
-  const Rw sc = (Rw)a.scale;
-#pragma unroll 1
-  for (int q = 0; q < NPROD; ++q) {
-    const cx<Rw>* ra = rs + ((long long)pp.a[q] * ROWS + rl) * M;
-    const cx<Rw>* rb = rs + ((long long)pp.b[q] * ROWS + rl) * M;
-    {
-      // forward step 1: radix R2 over k2 for this thread's n2' = t
-      cx<Rw> v[R2];
-#pragma unroll
-      for (int k2 = 0; k2 < R2; ++k2) v[k2] = rmul(ra[t + R1 * k2], rb[t + R1 * k2]);
-      DFT<R2, -1, Rw>::run(v);
-#pragma unroll
-      for (int k1p = 0; k1p < R2; ++k1p) exr[k1p * EXB + t] = v[k1p] * twM[(t * k1p) & (M - 1)];
-    }
-    __syncthreads();
-    if (t < R2) {
-      cx<Rw> v[R1];
-#pragma unroll
-      for (int n2p = 0; n2p < R1; ++n2p) v[n2p] = exr[t * EXB + n2p];
-      DFT<R1, -1, Rw>::run(v);
-#pragma unroll
-      for (int k2p = 0; k2p < R1; ++k2p) zr[t + R2 * k2p] = v[k2p];
-    }
-    __syncthreads();
-    if (ok) {
-      cx<Ro>* dst = reinterpret_cast<cx<Ro>*>(ps.dst[q]) + row * a.ds;
-      for (int k = t; k < a.nout; k += T) dst[k] = cvt<Ro>(sc * r2c_post<Rw>(zr, k, M, twN));
-      for (int k = a.nout + t; k < a.nfill; k += T) dst[k] = mkc<Ro>(0, 0);
-    }
-    __syncthreads();
-  }
-}
-
 // ------------------------------------------------------------------------------------------
-// Warp-per-row fused z-pass for M = N3/2 = 32 E (E in {1, 2, 4, 8}).
+// Warp-per-row fused z-pass for M = N3/2 = 32 E (E in {2, 4, 8}).
 //
 // Lane l holds the entries n = l + 32 j (j < E) of a row.  Inverse length-M DFT:
 //   radix-E DFT over j in registers, twiddle e^{+2 pi i l k1 / M}, then a 32-point DFT across

@@ -1,12 +1,13 @@
 // Dispatch of the z-pass (contiguous axis) c2r / r2c kernels and of the fused product z-pass.
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstdlib>
-
-#include <cmath>
 
 #include "tg_fft_launch.h"
 #include "tg_fft_zoct.cuh"
 #include "tg_fft_zoct64.cuh"
+#include "tg_fft_zrows.cuh"
 
 namespace tg {
 
@@ -81,23 +82,15 @@ cudaError_t run_z_prec(const ZLaunch& l, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------- fused product z-pass
-template <typename Ri, typename Ro, typename Rw, int R1, int R2, int NIN, int NPROD>
-cudaError_t run_zprod_fast(const ZProdLaunch& l, cudaStream_t s) {
-  constexpr int M = R1 * R2;
-  constexpr int TPB = (M >= 128) ? 128 : 256;
-  constexpr int ROWS = TPB / R1;
-  constexpr int EXA = R2 + 1, EXB = R1 + 1;
-  constexpr int EXS = (R1 * EXA > R2 * EXB) ? R1 * EXA : R2 * EXB;
-  const size_t smem = (size_t)(3 * M + ROWS * EXS + (size_t)ROWS * M * (1 + NIN)) * sizeof(cx<Rw>);
-  auto kern = k_z_prod<Ri, Ro, Rw, R1, R2, NIN, NPROD>;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
-  dim3 grid((unsigned)((l.a.nrows + ROWS - 1) / ROWS), 1, 1);
-  kern<<<grid, TPB, smem, s>>>(l.a, l.ps, l.pp);
+template <typename Rw, int V>
+cudaError_t run_zprod_rows(const ZProdLaunch& l, cudaStream_t s) {
+  const int nw = std::min(kZRowsWarps, std::max(l.nin, l.nprod));
+  const size_t smem = (size_t)l.nin * V * 32 * sizeof(cx<Rw>);
+  auto kern = k_z_prod_rows<Rw, V>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  if (e != cudaSuccess) return e;
+  kern<<<(unsigned)((l.a.nrows + 15) / 16), 32 * nw, smem, s>>>(l.a, l.ps, l.pp, l.nin, l.nprod);
   return cudaGetLastError();
 }
 
@@ -270,10 +263,10 @@ cudaError_t run_zprod_m(const ZProdLaunch& l, cudaStream_t s) {
   }
   if (l.M == 128 && zpass_net_enabled()) return run_zprod_net128<Ri, Ro, Rw, NIN, NPROD>(l, s);
   switch (l.M) {
-    case 4: return run_zprod_fast<Ri, Ro, Rw, 2, 2, NIN, NPROD>(l, s);
-    case 8: return run_zprod_fast<Ri, Ro, Rw, 4, 2, NIN, NPROD>(l, s);
-    case 16: return run_zprod_fast<Ri, Ro, Rw, 4, 4, NIN, NPROD>(l, s);
-    case 32: return run_zprod_warp<Ri, Ro, Rw, 1, NIN, NPROD>(l, s);
+    case 4: return run_zprod_rows<Rw, 2>(l, s);
+    case 8: return run_zprod_rows<Rw, 4>(l, s);
+    case 16: return run_zprod_rows<Rw, 8>(l, s);
+    case 32: return run_zprod_rows<Rw, 16>(l, s);
     case 64: return run_zprod_warp<Ri, Ro, Rw, 2, NIN, NPROD>(l, s);
     case 128: return run_zprod_warp<Ri, Ro, Rw, 4, NIN, NPROD>(l, s);
     case 256: return run_zprod_warp<Ri, Ro, Rw, 8, NIN, NPROD>(l, s);
