@@ -11,6 +11,8 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "tg_fft_dmma.cuh"
+#include "tg_fft_fold.cuh"
 #include "tg_fft_launch.h"
 #include "tg_fft_mixed.cuh"
 #include "tg_fft_tc.cuh"
@@ -306,7 +308,7 @@ cudaError_t run_r2r_mm(const AxisLaunch& l, const R2RArgs& r, cudaStream_t s, bo
   return cudaGetLastError();
 }
 
-// the register-tiled matrix product (k_axis_r2r_gemm) unless TG_R2R_GEMM=0
+// the folded register-tiled matrix product (k_axis_r2r_fold) unless TG_R2R_GEMM=0
 bool r2r_gemm_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("TG_R2R_GEMM");
@@ -315,43 +317,105 @@ bool r2r_gemm_enabled() {
   return on;
 }
 
-template <typename Ri, typename Ro, typename Rw, int RT>
-cudaError_t run_r2r_gemm_rt(const AxisLaunch& l, const R2RArgs& r, int nrows, int nin, cudaStream_t s) {
-  const int ntile = (nrows + RT - 1) / RT;
-  const size_t smem = (size_t)nin * RT * sizeof(Rw);
-  auto kern = k_axis_r2r_gemm<Ri, Ro, Rw, RT>;
+// every field's kind has its matrix (all of the same size and direction) and the launch maps all N
+// points to the stored coefficients or back
+bool r2r_foldable(const AxisLaunch& l, const R2RArgs& r, bool& fwd) {
+  if (!r2r_gemm_enabled()) return false;
+  const int nin = amap_count(l.a.in), nout = amap_count(l.a.out);
+  fwd = r.kind[0] <= 1;
+  for (int f = 0; f < l.nfields; ++f) {
+    const int k = r.kind[f];
+    if (k < 0 || k > 3 || (k <= 1) != fwd || !r.mat[k] || r.mat_rows[k] != nout || r.mat_cols[k] != nin || l.a.comb[f])
+      return false;
+  }
+  return (fwd ? nin : nout) == l.L && nin >= 1 && nout >= 1;
+}
+
+template <typename Ri, int RT, bool FWD>
+cudaError_t run_r2r_fold_rt(const AxisLaunch& l, const R2RArgs& r, int ntile, int steps, bool vec, cudaStream_t s) {
+  const size_t smem = (size_t)kFoldAhead * 2 * kFoldCols * sizeof(cx<Ri>) +
+                      (size_t)steps * ((RT + 3) / 4 * 8) * sizeof(float);
+  auto kern = vec ? k_axis_r2r_fold<Ri, RT, FWD, true> : k_axis_r2r_fold<Ri, RT, FWD, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;
-  dim3 grid((l.a.ncols + 127) / 128, l.nbatch, l.nfields * ntile);
-  kern<<<grid, 128, smem, s>>>(l.a, l.ps, r, ntile);
+  dim3 grid((l.a.ncols + kFoldCols - 1) / kFoldCols, l.nbatch, l.nfields * ntile);
+  kern<<<grid, kFoldThreads, smem, s>>>(l.a, l.ps, r, l.L, ntile);
   return cudaGetLastError();
 }
 
-// when every field's kind has its matrix (all of the same size); the row tile leaving the fewest
-// idle rows
-template <typename Ri, typename Ro, typename Rw>
-cudaError_t run_r2r_gemm(const AxisLaunch& l, const R2RArgs& r, cudaStream_t s, bool* used) {
+// FP32: row tiles of 22 pairs, or of 11 where those leave an SM without its two blocks (every tile
+// reads the inputs again, so the larger one where the grid allows)
+template <typename Ri>
+cudaError_t run_r2r_fold(const AxisLaunch& l, const R2RArgs& r, cudaStream_t s, bool* used) {
   *used = false;
-  if (!r2r_gemm_enabled()) return cudaSuccess;
-  const int nin = amap_count(l.a.in), nout = amap_count(l.a.out);
+  bool fwd;
+  if (!r2r_foldable(l, r, fwd)) return cudaSuccess;
+  const int nin = amap_count(l.a.in), nout = amap_count(l.a.out), N = l.L;
+  const int pairs = fwd ? (nout + 1) / 2 : (N + 1) / 2, steps = fwd ? (N + 1) / 2 : (nin + 1) / 2;
+  const long long blocks = (long long)((l.a.ncols + kFoldCols - 1) / kFoldCols) * l.nbatch * l.nfields * ((pairs + 21) / 22);
+  const int rt = blocks < 2 * 148 ? 11 : 22, ntile = (pairs + rt - 1) / rt;
+  bool vec = ((l.a.ncols | l.a.sr | l.a.dr | l.a.sb | l.a.db) & 1) == 0;
   for (int f = 0; f < l.nfields; ++f) {
-    const int k = r.kind[f];
-    if (k < 0 || k > 3 || !r.mat[k] || r.mat_rows[k] != nout || r.mat_cols[k] != nin) return cudaSuccess;
+    const uintptr_t sp = reinterpret_cast<uintptr_t>(l.ps.src[f]), dp = reinterpret_cast<uintptr_t>(l.ps.dst[f]);
+    if (sizeof(Ri) == 8 && (sp & 15)) return cudaSuccess;  // 16-byte copies of complex double columns
+    vec = vec && ((sp | dp) & 15) == 0;
   }
-  if (nin < 1 || nout < 1 || (size_t)l.nfields * ((nout + 21) / 22) > 65535) return cudaSuccess;
-  const int w43 = (nout + 42) / 43 * 43 - nout, w22 = (nout + 21) / 22 * 22 - nout;
+  if ((long long)l.nfields * ntile > 65535 || (size_t)steps * 48 * sizeof(float) > 96 * 1024) return cudaSuccess;
   *used = true;
-  if (w43 <= w22) return run_r2r_gemm_rt<Ri, Ro, Rw, 43>(l, r, nout, nin, s);
-  return run_r2r_gemm_rt<Ri, Ro, Rw, 22>(l, r, nout, nin, s);
+  if (rt == 22)
+    return fwd ? run_r2r_fold_rt<Ri, 22, true>(l, r, ntile, steps, vec, s)
+               : run_r2r_fold_rt<Ri, 22, false>(l, r, ntile, steps, vec, s);
+  return fwd ? run_r2r_fold_rt<Ri, 11, true>(l, r, ntile, steps, vec, s)
+             : run_r2r_fold_rt<Ri, 11, false>(l, r, ntile, steps, vec, s);
 }
 
-// FP32 forms: the x-pass contraction on the tensor cores (k_axis_r2r_tc, 3xTF32) when a field of
+template <int MT, bool FWD>
+cudaError_t run_r2r_dmma_mt(const AxisLaunch& l, const R2RArgs& r, int nrb, int nst, cudaStream_t s) {
+  const size_t smem = sizeof(double) * ((size_t)kDmStages * kDmStageD + (size_t)nst * (kDmPairs / 4) * 2 * MT * 32);
+  auto kern = k_axis_r2r_dmma<MT, FWD>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const int ntiles = (l.a.ncols + kDmCols - 1) / kDmCols;
+  const long long per = (long long)l.nbatch * l.nfields * nrb;
+  const int P = (int)std::max<long long>(1, std::min<long long>(ntiles, 148 / per));
+  dim3 grid(P, l.nbatch, l.nfields * nrb);
+  kern<<<grid, kDmThreads, smem, s>>>(l.a, l.ps, r, l.L, nrb);
+  return cudaGetLastError();
+}
+
+// FP64: the folded product on the matrix instructions.  Row tiles of 8 MT pairs with MT the smaller
+// of two values that needs no more row blocks than the larger (N1 = 129, 128: 6 forward, 9 inverse in
+// one block; N1 = 65: 3 and 5).
+cudaError_t run_r2r_dmma(const AxisLaunch& l, const R2RArgs& r, cudaStream_t s, bool* used) {
+  *used = false;
+  bool fwd;
+  if (!r2r_foldable(l, r, fwd)) return cudaSuccess;
+  const int nin = amap_count(l.a.in), nout = amap_count(l.a.out), N = l.L;
+  for (int f = 0; f < l.nfields; ++f)  // 16-byte copies
+    if (((reinterpret_cast<uintptr_t>(l.ps.src[f]) | reinterpret_cast<uintptr_t>(l.ps.dst[f])) & 15) != 0) return cudaSuccess;
+  const int pairs = fwd ? (nout + 1) / 2 : (N + 1) / 2, mts = (pairs + 7) / 8;
+  const int nst = ((fwd ? (N + 1) / 2 : (nin + 1) / 2) + kDmPairs - 1) / kDmPairs;
+  const int big = fwd ? 6 : 9, small = fwd ? 3 : 5;
+  const int mt = (mts + small - 1) / small <= (mts + big - 1) / big ? small : big;
+  const int nrb = (mts + mt - 1) / mt;
+  const size_t smem = sizeof(double) * ((size_t)kDmStages * kDmStageD + (size_t)nst * (kDmPairs / 4) * 2 * mt * 32);
+  if (smem > 227 * 1024 || (long long)l.nfields * nrb > 65535) return cudaSuccess;
+  *used = true;
+  if (fwd) return mt == 3 ? run_r2r_dmma_mt<3, true>(l, r, nrb, nst, s) : run_r2r_dmma_mt<6, true>(l, r, nrb, nst, s);
+  return mt == 5 ? run_r2r_dmma_mt<5, false>(l, r, nrb, nst, s) : run_r2r_dmma_mt<9, false>(l, r, nrb, nst, s);
+}
+
+// FP32 forms: the x-inverse contraction on the tensor cores (k_axis_r2r_tc, 3xTF32) when a field of
 // one request spans at least kTcMinTiles column tiles (the per-block set-up, coefficient pairs and
-// tensor memory, amortises; measured FP32-mixed steps against the register-tiled form: 129 x 256
-// x 256 1.89 against 2.92 ms, 65 x 128 x 128 0.342 against 0.397 ms).  The rule looks at one
-// request's geometry only, so a request batched in the serving loop takes the same path as on a
-// lone context.  TG_R2R_TC=0 never, =1 always.
+// tensor memory, amortises) and the folded product needs more than kTcMinPairs row pairs, three row
+// tiles of 22 that each read the inputs again.  Measured launches, tensor cores against folded:
+// inverse 129 x 256 x 256 56.4 / 70.1 us, 97 x 128 x 256 30.0 / 38.6, 65 x 256 x 128 23.7 / 20.1,
+// 65 x 128 x 128 19.4 / 17.1; forward 133.7 / 115.1, 54.0 / 52.0, 40.5 / 26.7, 26.1 / 16.6.  The rule
+// looks at one request's geometry only, so a request batched in the serving loop takes the same path
+// as on a lone context.  TG_R2R_TC=0 never, =1 always.
 constexpr int kTcMinTiles = 16;
+constexpr int kTcMinPairs = 45;
 int r2r_tc_mode() {
   static const int m = [] {
     const char* e = std::getenv("TG_R2R_TC");
@@ -367,7 +431,8 @@ cudaError_t run_r2r_tc(const AxisLaunch& l, const R2RArgs& r, cudaStream_t s, bo
   *used = false;
   const int mode = r2r_tc_mode();
   if (mode == 0) return cudaSuccess;
-  if (mode == 2 && (2LL * l.a.ncols + 127) / 128 < kTcMinTiles) return cudaSuccess;
+  if (mode == 2 && ((2LL * l.a.ncols + 127) / 128 < kTcMinTiles || r.kind[0] <= 1 || (l.L + 1) / 2 < kTcMinPairs))
+    return cudaSuccess;
   const int nin = amap_count(l.a.in), nout = amap_count(l.a.out);
   for (int f = 0; f < l.nfields; ++f) {
     const int k = r.kind[f];
@@ -413,9 +478,14 @@ cudaError_t run_r2r(const AxisLaunch& l, const R2RArgs& r, int N, cudaStream_t s
     cudaError_t e = run_r2r_tc<Ri>(l, r, s, &used);
     if (e != cudaSuccess || used) return e;
   }
-  {
+  if constexpr (sizeof(Rw) == 8) {
     bool used = false;
-    cudaError_t e = run_r2r_gemm<Ri, Ro, Rw>(l, r, s, &used);
+    cudaError_t e = run_r2r_dmma(l, r, s, &used);
+    if (e != cudaSuccess || used) return e;
+  }
+  if constexpr (sizeof(Ro) == 4 && sizeof(Rw) == 4) {
+    bool used = false;
+    cudaError_t e = run_r2r_fold<Ri>(l, r, s, &used);
     if (e != cudaSuccess || used) return e;
   }
   {

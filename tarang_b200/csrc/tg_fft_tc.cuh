@@ -1,7 +1,7 @@
 // The SCFT x-pass contraction Y[m][c] = scale * sum_k T[k][m] X[k][c] (T real, X complex) on the
 // 5th-generation tensor cores, for the FP32 forms: 3xTF32 (T = Th + Tl, X = Xh + Xl split into
 // TF32 pairs, Y ~ Th Xh + Th Xl + Tl Xh, FP32 accumulation), the sine/cosine transforms of
-// scft_tr.cc:440-639 as in k_axis_r2r_gemm.
+// scft_tr.cc:440-639 as in k_axis_r2r_fold, unfolded.
 //
 // The complex columns are read as real ones (re, im interleaved): a tile is 128 real columns, the
 // MMA's M dimension (A = the tile transposed, 128 x K); the output rows are the MMA's N dimension
