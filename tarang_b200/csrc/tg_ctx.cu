@@ -139,7 +139,10 @@ int max_radius_inside(const tg_ctx* c) {
 // X-inverse, Y-inverse, fused z-pass (c2r, products, r2c), Y-forward, X-forward.
 // inputs: compact fields of precision inprec.  MHD: in[0..2] = U, in[3..5] = B, the x-pass
 // forms z+ = U + B (fields 0..2) and z- = U - B (fields 3..5).
-int run_pipeline(tg_ctx* c, const void* const* in, int inprec) {
+// trace_free: the products without the third square, which is taken from the first two
+// (u1u1 - u3u3, u2u2 - u3u3; z+- alike): five products instead of six, eight instead of nine.  Only for a
+// right-hand side that is projected: the velocity's term changes by a gradient.
+int run_pipeline(tg_ctx* c, const void* const* in, int inprec, bool trace_free) {
   const void* src[6];
   const void* src2[6] = {};
   int comb[6] = {0, 0, 0, 0, 0, 0};
@@ -154,8 +157,29 @@ int run_pipeline(tg_ctx* c, const void* const* in, int inprec) {
   }
   int rc = pipe_inverse_xy(c, c->nin, src, src2, comb, inprec, c->nstate, c->WX, c->WY);
   if (rc) return rc;
-  return pipe_products_forward(c, c->nin, c->WY, c->nprod, c->pairs, c->PP, c->PY, c->PX);
+  if (!trace_free) return pipe_products_forward(c, c->nin, c->WY, c->nprod, c->pairs, c->PP, c->PY, c->PX);
+  ProdPairs pp{};
+  void *PP[8], *PY[8], *PX[8];
+  int kinds[8];
+  for (int q = 0; q < c->nprod - 1; ++q) {
+    const int o = q < 2 ? q : q + 1;
+    pp.a[q] = c->pairs.a[o];
+    pp.b[q] = c->pairs.b[o];
+    if (q < 2) {
+      pp.c[q] = c->pairs.a[2];
+      pp.d[q] = c->pairs.b[2];
+    }
+    PP[q] = c->PP[o];
+    PY[q] = c->PY[o];
+    PX[q] = c->PX[o];
+    kinds[q] = c->xfwd_kind[o];
+  }
+  return pipe_products_forward(c, c->nin, c->WY, c->nprod - 1, pp, PP, PY, PX, kinds);
 }
+
+// whether a step's products are trace-free: always, but for FP64 MHD rows of N3 = 256, whose z-pass has
+// no room for it (run_zprod_m)
+bool step_trace_free(const tg_ctx* c) { return !(c->phys == TG_MHD && c->tprec == F64 && c->Mz == 128); }
 
 // U: the c->nstate fields the force is computed from (the stage input)
 int run_force(tg_ctx* c, const void* const* U, int uprec) {
@@ -311,9 +335,11 @@ int run_stages(tg_ctx* c, int first, bool ring) {
     }
     int rc = run_force(c, in, inprec);
     if (rc) return rc;
-    rc = run_pipeline(c, in, inprec);
+    const bool tf = step_trace_free(c);
+    rc = run_pipeline(c, in, inprec, tf);
     if (rc) return rc;
     RKArgs a = rk_args(c, stage);
+    if (tf) a.PX[2] = nullptr;
     for (int i = 0; i < c->nstate; ++i) a.IN[i] = in[i];
     a.inprec = (inprec == F64) ? 0 : 1;
     {
@@ -321,7 +347,7 @@ int run_stages(tg_ctx* c, int first, bool ring) {
       // field written (1-3, 7) or U0 (final stages)
       const double ns = c->nstate, e = el_compact(c);
       const bool tot_rd = stage >= 2 && stage <= 4, tot_wr = stage >= 1 && stage <= 3;
-      const double rd = c->nprod * e * c->tsz + ns * e * 16 + (tot_rd ? ns * e * 16 : 0);
+      const double rd = (c->nprod - (tf ? 1 : 0)) * e * c->tsz + ns * e * 16 + (tot_rd ? ns * e * 16 : 0);
       const double wr = (stage_is_final(stage) ? ns * e * 16 : ns * e * c->tsz) + (tot_wr ? ns * e * 16 : 0);
       ProfScope pr(c, "rk_stage", rd + wr);
       TG_CK(launch_rk(a, c->phys, c->tprec, c->tprec, 0, c->st, nullptr));
@@ -1402,7 +1428,7 @@ int tg_compute_nlin(tg_ctx* c) {
   cudaSetDevice(c->dev);
   const void* in[6];
   for (int i = 0; i < c->nstate; ++i) in[i] = c->U0[i];
-  int rc = run_pipeline(c, in, F64);
+  int rc = run_pipeline(c, in, F64, false);
   if (rc) return rc;
   TG_CK(launch_assemble_nlin(c->g, c->phys, c->tprec, (const void* const*)c->PX, c->NL, c->st));
   c->have_nlin = true;

@@ -26,7 +26,7 @@ struct tg_ctx {
   long long S = 0;          // compact elements per field
   long long D = 0;          // dense elements per field
   int nstate = 3, nin = 3, nprod = 6;
-  tg::ProdPairs pairs{};
+  tg::ProdPairs pairs;
   double nu_of[6] = {0, 0, 0, 0, 0, 0};
   double nuh_of[6] = {0, 0, 0, 0, 0, 0};  // hyper coefficients per state field (0: off)
   // batch of same-shape requests (serving): B slots, the first nact of them advanced by a step;

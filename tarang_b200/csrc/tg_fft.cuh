@@ -463,8 +463,10 @@ __global__ void __launch_bounds__(128) k_z_r2c_dft(ZArgs a, PtrSet ps, int M) {
 // The forward FFT runs the inverse's steps backwards, so a thread's real-space positions are the
 // ones it needs again and the products are formed without another exchange.
 // ------------------------------------------------------------------------------------------
+// product q = r[a] r[b], less r[c] r[d] where c >= 0
 struct ProdPairs {
   signed char a[12], b[12];
+  signed char c[12] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1}, d[12];
 };
 
 // ------------------------------------------------------------------------------------------
@@ -587,10 +589,15 @@ __global__ void __launch_bounds__(32 * WPB, (E <= 4 ? (sizeof(Rw) == 8 ? 4 : 6) 
     // ---- products and forward (r2c)
 #pragma unroll 1
     for (int q = 0; q < NPROD; ++q) {
-      const int pa = pp.a[q], pb = pp.b[q];
+      const int pa = pp.a[q], pb = pp.b[q], pc = pp.c[q], pd = pp.d[q];
       cx<Rw> v[E];
 #pragma unroll
       for (int k1 = 0; k1 < E; ++k1) v[k1] = rmul(rs[(pa * E + k1) * 32 + lane], rs[(pb * E + k1) * 32 + lane]);
+      if (pc >= 0) {
+#pragma unroll
+        for (int k1 = 0; k1 < E; ++k1)
+          v[k1] = v[k1] - rmul(rs[(pc * E + k1) * 32 + lane], rs[(pd * E + k1) * 32 + lane]);
+      }
       lane_dit32_fwd<Rw, E>(v, tws, lane);
 #pragma unroll
       for (int k1 = 1; k1 < E; ++k1) v[k1] = v[k1] * conjc(tw1[k1]);
@@ -828,10 +835,15 @@ __global__ void __launch_bounds__(32 * WPB, sizeof(Rw) == 8 ? 4 : 6)
     // at the 80-register bound: z-pass 209 -> 200 us at 256^3), rolled in FP64 (no gain there)
 #pragma unroll (sizeof(Rw) == 4 ? NPROD : 1)
     for (int q = 0; q < NPROD; ++q) {
-      const int pa = pp.a[q], pb = pp.b[q];
+      const int pa = pp.a[q], pb = pp.b[q], pc = pp.c[q], pd = pp.d[q];
       cx<Rw> v[E];
 #pragma unroll
       for (int k1 = 0; k1 < E; ++k1) v[k1] = rmul(rs[(pa * E + k1) * 32 + lane], rs[(pb * E + k1) * 32 + lane]);
+      if (pc >= 0) {
+#pragma unroll
+        for (int k1 = 0; k1 < E; ++k1)
+          v[k1] = v[k1] - rmul(rs[(pc * E + k1) * 32 + lane], rs[(pd * E + k1) * 32 + lane]);
+      }
       net.fwd(v);
       net.phase_in(v, true);
       cx<Ro>* dst = reinterpret_cast<cx<Ro>*>(ps.dst[q]) + row * a.ds;

@@ -165,35 +165,39 @@ bool zpass_oct_enabled() {
   return v == 1;
 }
 
-// the physics layout k_z_prod_oct hard-codes (OctLayout), if the launch's product pairs are it
+// the physics layout k_z_prod_oct hard-codes (OctLayout), if the launch's products are it; tf: its
+// trace-free form
 template <int NIN, int NPROD>
-int oct_phys(const ProdPairs& pp) {
+int oct_phys(const ProdPairs& pp, bool& tf) {
   static const signed char F_A[6] = {0, 1, 2, 0, 1, 2}, F_B[6] = {0, 1, 2, 1, 2, 0};
   static const signed char M_A[9] = {0, 1, 2, 0, 3, 1, 4, 2, 5}, M_B[9] = {3, 4, 5, 4, 1, 5, 2, 3, 0};
   static const signed char S_A[9] = {0, 1, 2, 0, 1, 2, 0, 1, 2}, S_B[9] = {0, 1, 2, 1, 2, 0, 3, 3, 3};
   static const signed char E_A[9] = {3, 3, 3, 4, 4, 4, 5, 5, 5}, E_B[9] = {0, 1, 2, 0, 1, 2, 0, 1, 2};
   const signed char *A, *B;
   int ph;
-  if (NIN == 3 && NPROD == 6) {
+  tf = NPROD == 5 || NPROD == 8;
+  if (NIN == 3) {
     A = F_A, B = F_B, ph = 0;
-  } else if (NIN == 6 && NPROD == 9) {
+  } else if (NIN == 6) {
     if (pp.a[0] == 0) A = M_A, B = M_B, ph = 1;
     else A = E_A, B = E_B, ph = 3;
-  } else if (NIN == 4 && NPROD == 9) {
-    A = S_A, B = S_B, ph = 2;
   } else {
-    return -1;
+    A = S_A, B = S_B, ph = 2;
   }
-  for (int q = 0; q < NPROD; ++q)
-    if (pp.a[q] != A[q] || pp.b[q] != B[q]) return -1;
+  for (int q = 0; q < NPROD; ++q) {
+    const int o = tf && q >= 2 ? q + 1 : q;  // the third square is left out
+    if (pp.a[q] != A[o] || pp.b[q] != B[o]) return -1;
+    const bool less = tf && q < 2;
+    if ((pp.c[q] >= 0) != less || (less && (pp.c[q] != A[2] || pp.d[q] != B[2]))) return -1;
+  }
   return ph;
 }
 
-template <typename Ri, typename Ro, typename Rw, int PHYS, bool PRUNE>
+template <typename Ri, typename Ro, typename Rw, int PHYS, bool PRUNE, bool TF>
 cudaError_t run_zprod_oct(const ZProdLaunch& l, cudaStream_t s) {
   constexpr int WPB = 4;
-  const size_t smem = sizeof(cx<Rw>) * ((size_t)kOctEntries * 8 + (size_t)WPB * OctLayout<PHYS>::npark * 16 * 32);
-  auto kern = k_z_prod_oct<Ri, Ro, Rw, PHYS, PRUNE>;
+  const size_t smem = sizeof(cx<Rw>) * ((size_t)kOctEntries * 8 + (size_t)WPB * (OctLayout<PHYS>::npark + (PHYS == 1 && TF)) * 16 * 32);
+  auto kern = k_z_prod_oct<Ri, Ro, Rw, PHYS, PRUNE, TF>;
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -209,20 +213,17 @@ cudaError_t run_zprod_oct(const ZProdLaunch& l, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-template <typename Ri, typename Ro, typename Rw, int NIN, int NPROD>
-cudaError_t run_zprod_oct_any(const ZProdLaunch& l, int ph, cudaStream_t s) {
-  const bool prune = l.a.nin <= 96 && l.a.nout <= 96;
-  if (ph == 0) return prune ? run_zprod_oct<Ri, Ro, Rw, 0, true>(l, s) : run_zprod_oct<Ri, Ro, Rw, 0, false>(l, s);
-  if (ph == 1) return prune ? run_zprod_oct<Ri, Ro, Rw, 1, true>(l, s) : run_zprod_oct<Ri, Ro, Rw, 1, false>(l, s);
-  if (ph == 3) return prune ? run_zprod_oct<Ri, Ro, Rw, 3, true>(l, s) : run_zprod_oct<Ri, Ro, Rw, 3, false>(l, s);
-  return prune ? run_zprod_oct<Ri, Ro, Rw, 2, true>(l, s) : run_zprod_oct<Ri, Ro, Rw, 2, false>(l, s);
+template <typename Ri, typename Ro, typename Rw, int PHYS, bool TF>
+cudaError_t run_zprod_oct_any(const ZProdLaunch& l, cudaStream_t s) {
+  if (l.a.nin <= 96 && l.a.nout <= 96) return run_zprod_oct<Ri, Ro, Rw, PHYS, true, TF>(l, s);
+  return run_zprod_oct<Ri, Ro, Rw, PHYS, false, TF>(l, s);
 }
 
-template <typename Ri, typename Ro, typename Rw, int PHYS, bool PRUNE>
+template <typename Ri, typename Ro, typename Rw, int PHYS, bool PRUNE, bool TF>
 cudaError_t run_zprod_oct64(const ZProdLaunch& l, cudaStream_t s) {
   constexpr int WPB = 4;
-  const size_t smem = sizeof(cx<Rw>) * ((size_t)kO64Entries * 8 + (size_t)WPB * OctLayout<PHYS>::npark * 8 * 32);
-  auto kern = k_z_prod_oct64<Ri, Ro, Rw, PHYS, PRUNE>;
+  const size_t smem = sizeof(cx<Rw>) * ((size_t)kO64Entries * 8 + (size_t)WPB * (OctLayout<PHYS>::npark + (PHYS == 1 && TF)) * 8 * 32);
+  auto kern = k_z_prod_oct64<Ri, Ro, Rw, PHYS, PRUNE, TF>;
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -238,28 +239,35 @@ cudaError_t run_zprod_oct64(const ZProdLaunch& l, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-template <typename Ri, typename Ro, typename Rw, int NIN, int NPROD>
-cudaError_t run_zprod_oct64_any(const ZProdLaunch& l, int ph, cudaStream_t s) {
-  const bool prune = l.a.nin <= 48 && l.a.nout <= 48;
-  if (ph == 0) return prune ? run_zprod_oct64<Ri, Ro, Rw, 0, true>(l, s) : run_zprod_oct64<Ri, Ro, Rw, 0, false>(l, s);
-  if (ph == 1) return prune ? run_zprod_oct64<Ri, Ro, Rw, 1, true>(l, s) : run_zprod_oct64<Ri, Ro, Rw, 1, false>(l, s);
-  if (ph == 3) return prune ? run_zprod_oct64<Ri, Ro, Rw, 3, true>(l, s) : run_zprod_oct64<Ri, Ro, Rw, 3, false>(l, s);
-  return prune ? run_zprod_oct64<Ri, Ro, Rw, 2, true>(l, s) : run_zprod_oct64<Ri, Ro, Rw, 2, false>(l, s);
+template <typename Ri, typename Ro, typename Rw, int PHYS, bool TF>
+cudaError_t run_zprod_oct64_any(const ZProdLaunch& l, cudaStream_t s) {
+  if (l.a.nin <= 48 && l.a.nout <= 48) return run_zprod_oct64<Ri, Ro, Rw, PHYS, true, TF>(l, s);
+  return run_zprod_oct64<Ri, Ro, Rw, PHYS, false, TF>(l, s);
 }
 
 template <typename Ri, typename Ro, typename Rw, int NIN, int NPROD>
 cudaError_t run_zprod_m(const ZProdLaunch& l, cudaStream_t s) {
+  constexpr bool kTf = NPROD == 5 || NPROD == 8;
+  constexpr int kPh = NIN == 3 ? 0 : (NIN == 6 ? 1 : 2);
+  bool tf;
   if (l.M == 64 && l.a.oct && zpass_oct_enabled() && l.a.nin <= 65 && l.a.nout <= 65) {
-    const int ph = oct_phys<NIN, NPROD>(l.pp);
-    if (ph >= 0) return run_zprod_oct64_any<Ri, Ro, Rw, NIN, NPROD>(l, ph, s);
+    const int ph = oct_phys<NIN, NPROD>(l.pp, tf);
+    if (ph == kPh) return run_zprod_oct64_any<Ri, Ro, Rw, kPh, kTf>(l, s);
+    if constexpr (NIN == 6 && !kTf)
+      if (ph == 3) return run_zprod_oct64_any<Ri, Ro, Rw, 3, false>(l, s);
   }
-  if (l.M == 128 && l.a.oct && zpass_oct_enabled() && l.a.nin <= 129 && l.a.nout <= 129) {
+  // the fourth parked row of the trace-free MHD form does not fit two FP64 blocks of k_z_prod_oct an SM
+  constexpr bool kNoOct = NIN == 6 && kTf && sizeof(Rw) == 8;
+  if (!kNoOct && l.M == 128 && l.a.oct && zpass_oct_enabled() && l.a.nin <= 129 && l.a.nout <= 129) {
     // the paired output stores need even row strides and 2-entry-aligned product buffers
     bool aligned = (l.a.ds % 2) == 0;
     for (int q = 0; q < NPROD && aligned; ++q)
       aligned = (reinterpret_cast<uintptr_t>(l.ps.dst[q]) % (2 * sizeof(cx<Ro>))) == 0;
-    const int ph = aligned ? oct_phys<NIN, NPROD>(l.pp) : -1;
-    if (ph >= 0) return run_zprod_oct_any<Ri, Ro, Rw, NIN, NPROD>(l, ph, s);
+    const int ph = aligned ? oct_phys<NIN, NPROD>(l.pp, tf) : -1;
+    if constexpr (!kNoOct)
+      if (ph == kPh) return run_zprod_oct_any<Ri, Ro, Rw, kPh, kTf>(l, s);
+    if constexpr (NIN == 6 && !kTf)
+      if (ph == 3) return run_zprod_oct_any<Ri, Ro, Rw, 3, false>(l, s);
   }
   if (l.M == 128 && zpass_net_enabled()) return run_zprod_net128<Ri, Ro, Rw, NIN, NPROD>(l, s);
   switch (l.M) {
@@ -279,6 +287,9 @@ cudaError_t run_zprod_prec(const ZProdLaunch& l, cudaStream_t s) {
   if (l.nin == 3 && l.nprod == 6) return run_zprod_m<Ri, Ro, Rw, 3, 6>(l, s);
   if (l.nin == 6 && l.nprod == 9) return run_zprod_m<Ri, Ro, Rw, 6, 9>(l, s);
   if (l.nin == 4 && l.nprod == 9) return run_zprod_m<Ri, Ro, Rw, 4, 9>(l, s);
+  if (l.nin == 3 && l.nprod == 5) return run_zprod_m<Ri, Ro, Rw, 3, 5>(l, s);
+  if (l.nin == 6 && l.nprod == 8) return run_zprod_m<Ri, Ro, Rw, 6, 8>(l, s);
+  if (l.nin == 4 && l.nprod == 8) return run_zprod_m<Ri, Ro, Rw, 4, 8>(l, s);
   return cudaErrorInvalidValue;
 }
 

@@ -66,6 +66,8 @@ __device__ __forceinline__ cx<R> cmul_conjb(cx<R> a, cx<R> b) {  // a conj(b)
 //   1 MHD     inputs z+1..3 (parked), z-1..3 (registers); PA = {0,1,2,0,3,1,4,2,5},
 //             PB = {3,4,5,4,1,5,2,3,0}: each product pairs one z+ with one z-
 //   2 scalar  inputs u1 u2 u3 (parked), theta (registers); products as fluid, then u_i theta
+//   TF (trace-free): the third square is taken from the first two and left out (fluid u1u1 - u3u3,
+//     u2u2 - u3u3, then as above; MHD the same of z+i z-i), for a right-hand side that is projected
 //   3 energy transfer  inputs H1..3 (parked), G1..3 (registers); product 3 i + j = G_i H_j (tg_et.cu)
 template <int PHYS>
 struct OctLayout {
@@ -418,14 +420,14 @@ struct OctOcc {
   static constexpr int v = sizeof(Rw) == 8 ? 2 : (PHYS == 0 ? 4 : 3);
 };
 
-template <typename Ri, typename Ro, typename Rw, int PHYS, bool PRUNE>
+template <typename Ri, typename Ro, typename Rw, int PHYS, bool PRUNE, bool TF>
 __global__ void __launch_bounds__(128, OctOcc<Rw, PHYS>::v) k_z_prod_oct(ZArgs a, PtrSet ps) {
   using Lay = OctLayout<PHYS>;
-  constexpr int NP = Lay::npark;
+  constexpr int NP = Lay::npark, NR = NP + (PHYS == 1 && TF ? 1 : 0);  // parked rows: inputs (and z+3 z-3)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cx<Rw>* tab = reinterpret_cast<cx<Rw>*>(smem_raw);
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  cx<Rw>* rs = tab + kOctEntries * 8 + (size_t)wib * NP * 16 * 32;
+  cx<Rw>* rs = tab + kOctEntries * 8 + (size_t)wib * NR * 16 * 32;
   const Rw sc = (Rw)a.scale;
   for (int i = threadIdx.x; i < kOctEntries * 8; i += blockDim.x) {
     cx<Rw> v = cvt<Rw>(a.oct[i]);
@@ -466,13 +468,22 @@ __global__ void __launch_bounds__(128, OctOcc<Rw, PHYS>::v) k_z_prod_oct(ZArgs a
     if constexpr (PHYS == 0 || PHYS == 2) {
       // products of two parked inputs
 #pragma unroll 1
-      for (int q = 0; q < 6; ++q) {
-        const int pa = q < 3 ? q : q - 3, pb = q < 3 ? q : (q == 5 ? 0 : q - 2);
+      for (int q = 0; q < (TF ? 5 : 6); ++q) {
+        // the squares (TF: the first two, less the third), then 1 2, 2 3, 3 1
+        constexpr int SQ = TF ? 2 : 3;
+        const int pa = q < SQ ? q : q - SQ, pb = q < SQ ? q : (q == SQ + 2 ? 0 : q - SQ + 1);
         cx<Rw> v[16];
 #pragma unroll
         for (int s = 0; s < 16; ++s) {
           const cx<Rw> x = rs[(pa * 16 + s) * 32 + lane];
           v[s] = (pa == pb) ? rmul(x, x) : rmul(x, rs[(pb * 16 + s) * 32 + lane]);
+        }
+        if (TF && q < SQ) {
+#pragma unroll
+          for (int s = 0; s < 16; ++s) {
+            const cx<Rw> x = rs[(2 * 16 + s) * 32 + lane];
+            v[s] = v[s] - rmul(x, x);
+          }
         }
         cx<Ro>* Y = live ? reinterpret_cast<cx<Ro>*>(ps.dst[q]) + row * a.ds : nullptr;
         L.template forward<Ro, PRUNE>(v, Y, a.nout, a.nfill);
@@ -481,7 +492,9 @@ __global__ void __launch_bounds__(128, OctOcc<Rw, PHYS>::v) k_z_prod_oct(ZArgs a
     if constexpr (PHYS != 0) {
       // register inputs, each multiplied with the three parked inputs
 #pragma unroll 1
-      for (int c = 3; c < Lay::nin; ++c) {
+      for (int ci = 3; ci < Lay::nin; ++ci) {
+        // TF MHD takes z-3 first: its product with z+3 is parked and taken from the other two squares
+        const int c = PHYS == 1 && TF ? (ci == 3 ? 5 : ci - 1) : ci;
         const cx<Ri>* X = live ? reinterpret_cast<const cx<Ri>*>(ps.src[c]) + row * a.ss : nullptr;
         cx<Rw> w[16];
         L.template inverse<Ri, PRUNE>(X, a.nin, w);
@@ -489,7 +502,7 @@ __global__ void __launch_bounds__(128, OctOcc<Rw, PHYS>::v) k_z_prod_oct(ZArgs a
         for (int j = 0; j < 3; ++j) {
           // PHYS 2: product 6 + j = u_j theta; PHYS 3: product 3 i + j = H_j G_i; PHYS 1: the three
           // products of z-(c) in order
-          int q = (PHYS == 3 ? 3 * (c - 3) : 6) + j, pa = j;
+          int q = (PHYS == 3 ? 3 * (c - 3) : (TF ? 5 : 6)) + j, pa = j;
           if constexpr (PHYS == 1) {
             const int sh = 4 * (3 * (c - 3) + j);
             q = (int)((kOctMhdQ >> sh) & 15);
@@ -498,6 +511,19 @@ __global__ void __launch_bounds__(128, OctOcc<Rw, PHYS>::v) k_z_prod_oct(ZArgs a
           cx<Rw> v[16];
 #pragma unroll
           for (int s = 0; s < 16; ++s) v[s] = rmul(rs[(pa * 16 + s) * 32 + lane], w[s]);
+          if constexpr (PHYS == 1 && TF) {
+            if (q == 2) {
+#pragma unroll
+              for (int s = 0; s < 16; ++s) rs[(3 * 16 + s) * 32 + lane] = v[s];
+              continue;
+            }
+            if (q < 2) {
+#pragma unroll
+              for (int s = 0; s < 16; ++s) v[s] = v[s] - rs[(3 * 16 + s) * 32 + lane];
+            } else {
+              --q;
+            }
+          }
           cx<Ro>* Y = live ? reinterpret_cast<cx<Ro>*>(ps.dst[q]) + row * a.ds : nullptr;
           L.template forward<Ro, PRUNE>(v, Y, a.nout, a.nfill);
         }

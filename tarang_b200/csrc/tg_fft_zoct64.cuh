@@ -218,14 +218,14 @@ struct Oct64Occ {
   static constexpr int v = sizeof(Rw) == 8 ? 3 : 4;
 };
 
-template <typename Ri, typename Ro, typename Rw, int PHYS, bool PRUNE>
+template <typename Ri, typename Ro, typename Rw, int PHYS, bool PRUNE, bool TF>
 __global__ void __launch_bounds__(128, Oct64Occ<Rw, PHYS>::v) k_z_prod_oct64(ZArgs a, PtrSet ps) {
   using Lay = OctLayout<PHYS>;
-  constexpr int NP = Lay::npark;
+  constexpr int NP = Lay::npark, NR = NP + (PHYS == 1 && TF ? 1 : 0);  // parked rows: inputs (and z+3 z-3)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cx<Rw>* tab = reinterpret_cast<cx<Rw>*>(smem_raw);
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  cx<Rw>* rs = tab + kO64Entries * 8 + (size_t)wib * NP * 8 * 32;
+  cx<Rw>* rs = tab + kO64Entries * 8 + (size_t)wib * NR * 8 * 32;
   const Rw sc = (Rw)a.scale;
   for (int i = threadIdx.x; i < kO64Entries * 8; i += blockDim.x) {
     cx<Rw> v = cvt<Rw>(a.oct[i]);
@@ -265,13 +265,22 @@ __global__ void __launch_bounds__(128, Oct64Occ<Rw, PHYS>::v) k_z_prod_oct64(ZAr
     if constexpr (PHYS == 0 || PHYS == 2) {
       // products of two parked inputs
 #pragma unroll 1
-      for (int q = 0; q < 6; ++q) {
-        const int pa = q < 3 ? q : q - 3, pb = q < 3 ? q : (q == 5 ? 0 : q - 2);
+      for (int q = 0; q < (TF ? 5 : 6); ++q) {
+        // the squares (TF: the first two, less the third), then 1 2, 2 3, 3 1
+        constexpr int SQ = TF ? 2 : 3;
+        const int pa = q < SQ ? q : q - SQ, pb = q < SQ ? q : (q == SQ + 2 ? 0 : q - SQ + 1);
         cx<Rw> v[8];
 #pragma unroll
         for (int s = 0; s < 8; ++s) {
           const cx<Rw> x = rs[(pa * 8 + s) * 32 + lane];
           v[s] = (pa == pb) ? rmul(x, x) : rmul(x, rs[(pb * 8 + s) * 32 + lane]);
+        }
+        if (TF && q < SQ) {
+#pragma unroll
+          for (int s = 0; s < 8; ++s) {
+            const cx<Rw> x = rs[(2 * 8 + s) * 32 + lane];
+            v[s] = v[s] - rmul(x, x);
+          }
         }
         cx<Ro>* Y = live ? reinterpret_cast<cx<Ro>*>(ps.dst[q]) + row * a.ds : nullptr;
         L.template forward<Ro, PRUNE>(v, Y, a.nout, a.nfill);
@@ -280,7 +289,9 @@ __global__ void __launch_bounds__(128, Oct64Occ<Rw, PHYS>::v) k_z_prod_oct64(ZAr
     if constexpr (PHYS != 0) {
       // register inputs, each multiplied with the three parked inputs
 #pragma unroll 1
-      for (int c = 3; c < Lay::nin; ++c) {
+      for (int ci = 3; ci < Lay::nin; ++ci) {
+        // TF MHD takes z-3 first: its product with z+3 is parked and taken from the other two squares
+        const int c = PHYS == 1 && TF ? (ci == 3 ? 5 : ci - 1) : ci;
         const cx<Ri>* X = live ? reinterpret_cast<const cx<Ri>*>(ps.src[c]) + row * a.ss : nullptr;
         cx<Rw> w[8];
         L.template inverse<Ri, PRUNE>(X, a.nin, w);
@@ -288,7 +299,7 @@ __global__ void __launch_bounds__(128, Oct64Occ<Rw, PHYS>::v) k_z_prod_oct64(ZAr
         for (int j = 0; j < 3; ++j) {
           // PHYS 2: product 6 + j = u_j theta; PHYS 3: product 3 i + j = H_j G_i; PHYS 1: the three
           // products of z-(c) in order
-          int q = (PHYS == 3 ? 3 * (c - 3) : 6) + j, pa = j;
+          int q = (PHYS == 3 ? 3 * (c - 3) : (TF ? 5 : 6)) + j, pa = j;
           if constexpr (PHYS == 1) {
             const int sh = 4 * (3 * (c - 3) + j);
             q = (int)((kOctMhdQ >> sh) & 15);
@@ -297,6 +308,19 @@ __global__ void __launch_bounds__(128, Oct64Occ<Rw, PHYS>::v) k_z_prod_oct64(ZAr
           cx<Rw> v[8];
 #pragma unroll
           for (int s = 0; s < 8; ++s) v[s] = rmul(rs[(pa * 8 + s) * 32 + lane], w[s]);
+          if constexpr (PHYS == 1 && TF) {
+            if (q == 2) {
+#pragma unroll
+              for (int s = 0; s < 8; ++s) rs[(3 * 8 + s) * 32 + lane] = v[s];
+              continue;
+            }
+            if (q < 2) {
+#pragma unroll
+              for (int s = 0; s < 8; ++s) v[s] = v[s] - rs[(3 * 8 + s) * 32 + lane];
+            } else {
+              --q;
+            }
+          }
           cx<Ro>* Y = live ? reinterpret_cast<cx<Ro>*>(ps.dst[q]) + row * a.ds : nullptr;
           L.template forward<Ro, PRUNE>(v, Y, a.nout, a.nfill);
         }

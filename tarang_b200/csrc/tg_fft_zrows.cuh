@@ -119,6 +119,12 @@ __global__ void __launch_bounds__(32 * kZRowsWarps)
     cx<Rw> v[V];
 #pragma unroll
     for (int k = 0; k < V; ++k) v[k] = rmul(xa[k * 32], xb[k * 32]);
+    if (pp.c[q] >= 0) {
+      const cx<Rw>* xc = rs + pp.c[q] * V * 32 + lane;
+      const cx<Rw>* xd = rs + pp.d[q] * V * 32 + lane;
+#pragma unroll
+      for (int k = 0; k < V; ++k) v[k] = v[k] - rmul(xc[k * 32], xd[k * 32]);
+    }
     L.lane_bfly(v);
     L.template lane_tws<-1, 1>(v);
     DFT<V, -1, Rw>::run(v);

@@ -86,6 +86,8 @@ __global__ void k_compact_to_dense(Geo g, const cx<R>* __restrict__ comp, cx<dou
 //  MHD   : 0 zp1zm1, 1 zp2zm2, 2 zp3zm3, 3 zp1zm2 (v1), 4 zm1zp2 (w1), 5 zp2zm3 (v2),
 //          6 zm2zp3 (w2), 7 zp3zm1 (v3), 8 zm3zp1 (w3)              (RSprod.cc:117-194)
 //  scalar: fluid 0..5, then 6 u1 th, 7 u2 th, 8 u3 th               (compute_nlin_SF.cc)
+// Trace-free form (PX[2] null): the third square is left out and taken from the first two, which changes
+// the velocity's term by the gradient of it; the projection takes that gradient out again.
 // x-derivative of a coefficient (Xderiv universal_tr.cc:186-210): FOUR i kx; SCFT a real factor
 // by the parity of the series, cos -> sin: -kx (Xderiv_Cos_SCFT), sin -> cos: +kx
 // (Xderiv_Sin_SCFT, scft_tr.cc:649-672)
@@ -109,7 +111,8 @@ __device__ __forceinline__ void assemble(const void* const* PX, long long idx, c
   if constexpr (PHYS == PH_FLUID || PHYS == PH_SCALAR || PHYS == PH_RB) {
     // parities of the products (RV_Forward_transform_RSprod Rvf.cc:179-186): u1u1, u2u2, u3u3,
     // u2u3 cos; u1u2, u3u1 sin; and u1 th cos, u2 th, u3 th sin (compute_nlin_SF.cc:80-115)
-    const cx<double> p0 = ldc<Rp>(PX[0], idx), p1 = ldc<Rp>(PX[1], idx), p2 = ldc<Rp>(PX[2], idx);
+    const cx<double> p0 = ldc<Rp>(PX[0], idx), p1 = ldc<Rp>(PX[1], idx);
+    const cx<double> p2 = PX[2] ? ldc<Rp>(PX[2], idx) : mkc<double>(0, 0);
     const cx<double> p3 = ldc<Rp>(PX[3], idx), p4 = ldc<Rp>(PX[4], idx), p5 = ldc<Rp>(PX[5], idx);
     n[0] = dx.cos_in(p0) + iky_ikz(ky, kz, p3, p5);
     n[1] = dx.sin_in(p3) + iky_ikz(ky, kz, p1, p4);
@@ -122,7 +125,7 @@ __device__ __forceinline__ void assemble(const void* const* PX, long long idx, c
     const double kx = dx.kx;
     cx<double> p[9];
 #pragma unroll
-    for (int q = 0; q < 9; ++q) p[q] = ldc<Rp>(PX[q], idx);
+    for (int q = 0; q < 9; ++q) p[q] = (q != 2 || PX[2]) ? ldc<Rp>(PX[q], idx) : mkc<double>(0, 0);
     // Zp.nlin (n) and Zm.nlin (nw)
     const cx<double> n0 = ikdot(kx, ky, kz, p[0], p[3], p[8]);
     const cx<double> n1 = ikdot(kx, ky, kz, p[4], p[1], p[5]);
