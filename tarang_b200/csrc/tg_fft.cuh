@@ -48,6 +48,7 @@ struct AxisArgs {
 // ------------------------------------------------------------------------------------------
 template <typename Ri, typename Ro, typename Rw, int R1, int R2, int DIR>
 __global__ void __launch_bounds__(256) k_axis_c2c(AxisArgs a, PtrSet ps) {
+  pdl_wait();
   constexpr int L = R1 * R2;
   constexpr int W = 256 / R1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -129,6 +130,7 @@ struct R2RArgs {
 
 template <typename Ri, typename Ro, typename Rw>
 __global__ void __launch_bounds__(256) k_axis_r2r(AxisArgs a, PtrSet ps, R2RArgs r, int N) {
+  pdl_wait();
   constexpr int W = 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cx<Rw>* tr = reinterpret_cast<cx<Rw>*>(smem_raw);  // 4N
@@ -197,6 +199,7 @@ __global__ void __launch_bounds__(256) k_axis_r2r(AxisArgs a, PtrSet ps, R2RArgs
 // k step is a broadcast load of 4 coefficients, a load of its columns and 8 or 16 FMAs.
 template <typename Ri, typename Ro, typename Rw, int CW>
 __global__ void __launch_bounds__(256) k_axis_r2r_mm(AxisArgs a, PtrSet ps, R2RArgs r) {
+  pdl_wait();
   constexpr int TR = 4;
   constexpr int CL = CW / 32;  // columns per lane: 2 (64-column tiles) or 1 (32)
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -541,6 +544,7 @@ __device__ __forceinline__ void lane_dit32_fwd(cx<R> (&v)[E], const cx<R> (&wl)[
 template <typename Ri, typename Ro, typename Rw, int E, int NIN, int NPROD, int WPB>
 __global__ void __launch_bounds__(32 * WPB, (E <= 4 ? (sizeof(Rw) == 8 ? 4 : 6) : (sizeof(Rw) == 8 ? 3 : 4)))
     k_z_prod_warp(ZArgs a, PtrSet ps, ProdPairs pp) {
+  pdl_wait();
   constexpr int M = 32 * E;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
@@ -771,6 +775,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 template <typename Ri, typename Ro, typename Rw, int NIN, int NPROD, int WPB, int PF>
 __global__ void __launch_bounds__(32 * WPB, sizeof(Rw) == 8 ? 4 : 6)
     k_z_prod_net128(ZArgs a, PtrSet ps, ProdPairs pp, int np) {
+  pdl_wait();
   constexpr int M = 128, E = 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;

@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(TmaW<Rw>::v * R1, AxisOcc<Rw, TmaW<Rw>::v * R1
     mbar_init_fence();
   }
   __syncthreads();
+  pdl_wait();
   if (tid == 0) {
     const unsigned in_bytes = (unsigned)(W * CEi * 8) * (unsigned)nin_rows;
     mbar_arrive_expect_tx(bar, COMB ? 2 * in_bytes : in_bytes);
@@ -195,16 +196,16 @@ cudaError_t run_axis_tma(const AxisLaunch& l, cudaStream_t s, bool* used) {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e != cudaSuccess) return e;
-    kern<<<grid, NT, smem, s>>>(l.a, tm, nin_rows, nout_rows, (unsigned)tile);
+    e = launch_pdl(kern, grid, NT, smem, s, l.a, tm, nin_rows, nout_rows, (unsigned)tile);
   } else {
     auto kern = k_axis_tma<Ri, Ro, Rw, R1, R2, DIR, false>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e != cudaSuccess) return e;
-    kern<<<grid, NT, smem, s>>>(l.a, tm, nin_rows, nout_rows, (unsigned)tile);
+    e = launch_pdl(kern, grid, NT, smem, s, l.a, tm, nin_rows, nout_rows, (unsigned)tile);
   }
   *used = true;
-  return cudaGetLastError();
+  return e;
 }
 
 template <typename Ri, typename Ro, typename Rw, int R1, int R2, int DIR>
@@ -227,8 +228,7 @@ cudaError_t run_axis_fast(const AxisLaunch& l, cudaStream_t s) {
     attr = true;
   }
   dim3 grid((l.a.ncols + W - 1) / W, l.nbatch, l.nfields);
-  kern<<<grid, 256, smem, s>>>(l.a, l.ps);
-  return cudaGetLastError();
+  return launch_pdl(kern, grid, 256, smem, s, l.a, l.ps);
 }
 
 // lengths that are no power of two (or beyond the register-staged kernels): the mixed-radix
@@ -252,8 +252,8 @@ cudaError_t run_axis_mixed(const AxisLaunch& l, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid((l.a.ncols + W - 1) / W, l.nbatch, l.nfields);
-  kern<<<grid, threads, smem, s>>>(l.a, l.ps, p);
-  return cudaGetLastError();
+  e = launch_pdl(kern, grid, threads, smem, s, l.a, l.ps, p);
+  return e;
 }
 
 template <typename Ri, typename Ro, typename Rw, int DIR>
@@ -303,9 +303,9 @@ cudaError_t run_r2r_mm(const AxisLaunch& l, const R2RArgs& r, cudaStream_t s, bo
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid((l.a.ncols + cw - 1) / cw, l.nbatch, l.nfields);
-  kern<<<grid, 256, smem, s>>>(l.a, l.ps, r);
+  e = launch_pdl(kern, grid, 256, smem, s, l.a, l.ps, r);
   *used = true;
-  return cudaGetLastError();
+  return e;
 }
 
 // the folded register-tiled matrix product (k_axis_r2r_fold) unless TG_R2R_GEMM=0
@@ -340,8 +340,8 @@ cudaError_t run_r2r_fold_rt(const AxisLaunch& l, const R2RArgs& r, int ntile, in
   if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;
   dim3 grid((l.a.ncols + kFoldCols - 1) / kFoldCols, l.nbatch, l.nfields * ntile);
-  kern<<<grid, kFoldThreads, smem, s>>>(l.a, l.ps, r, l.L, ntile);
-  return cudaGetLastError();
+  e = launch_pdl(kern, grid, kFoldThreads, smem, s, l.a, l.ps, r, l.L, ntile);
+  return e;
 }
 
 // FP32: row tiles of 22 pairs, or of 11 where those leave an SM without its two blocks (every tile
@@ -380,8 +380,8 @@ cudaError_t run_r2r_dmma_mt(const AxisLaunch& l, const R2RArgs& r, int nrb, int 
   const long long per = (long long)l.nbatch * l.nfields * nrb;
   const int P = (int)std::max<long long>(1, std::min<long long>(ntiles, 148 / per));
   dim3 grid(P, l.nbatch, l.nfields * nrb);
-  kern<<<grid, kDmThreads, smem, s>>>(l.a, l.ps, r, l.L, nrb);
-  return cudaGetLastError();
+  e = launch_pdl(kern, grid, kDmThreads, smem, s, l.a, l.ps, r, l.L, nrb);
+  return e;
 }
 
 // FP64: the folded product on the matrix instructions.  Row tiles of 8 MT pairs with MT the smaller
@@ -467,8 +467,8 @@ cudaError_t run_r2r_tc(const AxisLaunch& l, const R2RArgs& r, cudaStream_t s, bo
   const int P = std::max(1, std::min(t.ntiles, 148 / per));
   *used = true;
   dim3 grid(P, l.nbatch, l.nfields);
-  kern<<<grid, kTcThreads, smem, s>>>(l.a, l.ps, r, t);
-  return cudaGetLastError();
+  e = launch_pdl(kern, grid, kTcThreads, smem, s, l.a, l.ps, r, t);
+  return e;
 }
 
 template <typename Ri, typename Ro, typename Rw>
@@ -499,8 +499,8 @@ cudaError_t run_r2r(const AxisLaunch& l, const R2RArgs& r, int N, cudaStream_t s
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid((l.a.ncols + 31) / 32, l.nbatch, l.nfields);
-  kern<<<grid, 256, smem, s>>>(l.a, l.ps, r, N);
-  return cudaGetLastError();
+  e = launch_pdl(kern, grid, 256, smem, s, l.a, l.ps, r, N);
+  return e;
 }
 
 }  // namespace

@@ -100,8 +100,6 @@ __global__ void __launch_bounds__(kDmThreads, 1) k_axis_r2r_dmma(AxisArgs a, Ptr
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-#pragma unroll
-  for (int it = 0; it < kDmStages - 1; ++it) copy_stage();
   // coefficients in fragment order: A(row gid, k tig).  A sine's even rows take the difference; the
   // middle point of an odd N has none
   const double* M = r.mat[kind];
@@ -115,6 +113,9 @@ __global__ void __launch_bounds__(kDmThreads, 1) k_axis_r2r_dmma(AxisArgs a, Ptr
     Af[e] = (j < npair && k < nin && row < (FWD ? nrows : H) && !mid) ? M[(size_t)k * nrows + row] : 0.0;
   }
 
+  pdl_wait();
+#pragma unroll
+  for (int it = 0; it < kDmStages - 1; ++it) copy_stage();
   double c[2][MT][2];
 #pragma unroll
   for (int h = 0; h < 2; ++h)

@@ -38,6 +38,7 @@ constexpr int kFoldAhead = 8;                // steps in the ring
 template <typename Ri, int RT, bool FWD, bool VEC>
 __global__ void __launch_bounds__(kFoldThreads, RT <= 11 ? 3 : 2)
     k_axis_r2r_fold(AxisArgs a, PtrSet ps, R2RArgs r, int N, int ntile) {
+  pdl_wait();
   constexpr int D = kFoldAhead;
   constexpr int RP = (RT + 3) / 4 * 4, TP = 2 * RP;  // c0 and c1 of a step, each a whole number of 16 bytes
   constexpr int NQ = (int)sizeof(cx<Ri>) / 8;        // 16-byte pieces of a thread's two columns

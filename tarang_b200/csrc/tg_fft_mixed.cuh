@@ -222,6 +222,7 @@ struct MixTile {
 template <typename Ri, typename Ro, typename Rw, int DIR>
 __global__ void __launch_bounds__(kMixThreads, sizeof(Rw) == 8 ? 4 : 6)
     k_axis_mixed(AxisArgs a, PtrSet ps, const __grid_constant__ MixPlan pl) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int L = pl.L, W = 1 << pl.wsh;
   cx<Rw>* tw = reinterpret_cast<cx<Rw>*>(smem_raw);

@@ -224,6 +224,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_axis_r2r_tc(AxisArgs a, PtrSe
   proxy_fence();
   tc_fence_before();
   __syncthreads();
+  pdl_wait();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const long long ncr = 2LL * a.ncols;  // real columns

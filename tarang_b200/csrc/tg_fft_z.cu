@@ -90,8 +90,7 @@ cudaError_t run_zprod_rows(const ZProdLaunch& l, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;
-  kern<<<(unsigned)((l.a.nrows + 15) / 16), 32 * nw, smem, s>>>(l.a, l.ps, l.pp, l.nin, l.nprod);
-  return cudaGetLastError();
+  return launch_pdl(kern, (unsigned)((l.a.nrows + 15) / 16), 32 * nw, smem, s, l.a, l.ps, l.pp, l.nin, l.nprod);
 }
 
 template <typename Ri, typename Ro, typename Rw, int E, int NIN, int NPROD>
@@ -107,8 +106,7 @@ cudaError_t run_zprod_warp(const ZProdLaunch& l, cudaStream_t s) {
   }
   long long blocks = (l.a.nrows + WPB - 1) / WPB;
   if (blocks > 148LL * 32) blocks = 148LL * 32;
-  kern<<<(unsigned)blocks, 32 * WPB, smem, s>>>(l.a, l.ps, l.pp);
-  return cudaGetLastError();
+  return launch_pdl(kern, (unsigned)blocks, 32 * WPB, smem, s, l.a, l.ps, l.pp);
 }
 
 // M = 128: the transposed lane network (k_z_prod_net128) unless TG_ZPASS_NET=0 selects the
@@ -136,8 +134,7 @@ cudaError_t run_zprod_net128_pf(const ZProdLaunch& l, int np, cudaStream_t s) {
   }
   long long blocks = (l.a.nrows + WPB - 1) / WPB;
   if (blocks > 148LL * 32) blocks = 148LL * 32;
-  kern<<<(unsigned)blocks, 32 * WPB, smem, s>>>(l.a, l.ps, l.pp, np);
-  return cudaGetLastError();
+  return launch_pdl(kern, (unsigned)blocks, 32 * WPB, smem, s, l.a, l.ps, l.pp, np);
 }
 
 // The prefetching form when its buffers fit beside the register-bound occupancy (at most four
@@ -209,8 +206,7 @@ cudaError_t run_zprod_oct(const ZProdLaunch& l, cudaStream_t s) {
   long long blocks = (nquad + WPB - 1) / WPB;
   const long long resident = 148LL * OctOcc<Rw, PHYS>::v;
   if (blocks > resident) blocks = resident;
-  kern<<<(unsigned)blocks, 32 * WPB, smem, s>>>(l.a, l.ps);
-  return cudaGetLastError();
+  return launch_pdl(kern, (unsigned)blocks, 32 * WPB, smem, s, l.a, l.ps);
 }
 
 template <typename Ri, typename Ro, typename Rw, int PHYS, bool TF>
@@ -235,8 +231,7 @@ cudaError_t run_zprod_oct64(const ZProdLaunch& l, cudaStream_t s) {
   long long blocks = (nquad + WPB - 1) / WPB;
   const long long resident = 148LL * Oct64Occ<Rw, PHYS>::v;
   if (blocks > resident) blocks = resident;
-  kern<<<(unsigned)blocks, 32 * WPB, smem, s>>>(l.a, l.ps);
-  return cudaGetLastError();
+  return launch_pdl(kern, (unsigned)blocks, 32 * WPB, smem, s, l.a, l.ps);
 }
 
 template <typename Ri, typename Ro, typename Rw, int PHYS, bool TF>

@@ -436,6 +436,7 @@ __global__ void __launch_bounds__(128, OctOcc<Rw, PHYS>::v) k_z_prod_oct(ZArgs a
     tab[i] = v;
   }
   __syncthreads();
+  pdl_wait();
   OctLane<Rw, sizeof(Rw) == 4 && PHYS == 0> L;
   L.tab = tab;
   L.p = lane & 7;

@@ -234,6 +234,7 @@ __global__ void __launch_bounds__(128, Oct64Occ<Rw, PHYS>::v) k_z_prod_oct64(ZAr
     tab[i] = v;
   }
   __syncthreads();
+  pdl_wait();
   OctLane64<Rw, sizeof(Rw) == 4 && PHYS == 0> L;
   L.tab = tab;
   L.p = lane & 7;

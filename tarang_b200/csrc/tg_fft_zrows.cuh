@@ -87,6 +87,7 @@ struct ZRowLane {
 template <typename Rw, int V>
 __global__ void __launch_bounds__(32 * kZRowsWarps)
     k_z_prod_rows(ZArgs a, PtrSet ps, ProdPairs pp, int nin, int nprod) {
+  pdl_wait();
   constexpr int M = 2 * V;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cx<Rw>* rs = reinterpret_cast<cx<Rw>*>(smem_raw);  // [nin][V][32]

@@ -187,6 +187,7 @@ struct RKOcc {
 // in flight together; exp(-nu a dt K^2) is evaluated once per distinct viscosity.
 template <typename Rp, typename Rs, int PHYS, int SRC, int STAGE>
 __global__ void __launch_bounds__(TPB, RKOcc<PHYS>::v) k_rk(RKArgs a) {
+  pdl_wait();
   constexpr int NS = NState<PHYS>::v;
   const Geo& g = a.g;
   double acc[6] = {0, 0, 0, 0, 0, 0};
@@ -324,24 +325,23 @@ cudaError_t run_rk_src(const RKArgs& a, int src, cudaStream_t s, int nblk) {
     // precomputed right-hand sides enter at a scheme's first stage only (Time_advance after
     // Compute_rhs): RK4 1, EULER 5, RK2 7
     switch (a.stage) {
-      case 1: k_rk<Rp, Rs, PHYS, 1, 1><<<grid, TPB, 0, s>>>(a); break;
-      case 5: k_rk<Rp, Rs, PHYS, 1, 5><<<grid, TPB, 0, s>>>(a); break;
-      case 7: k_rk<Rp, Rs, PHYS, 1, 7><<<grid, TPB, 0, s>>>(a); break;
+      case 1: return launch_pdl(k_rk<Rp, Rs, PHYS, 1, 1>, grid, TPB, 0, s, a);
+      case 5: return launch_pdl(k_rk<Rp, Rs, PHYS, 1, 5>, grid, TPB, 0, s, a);
+      case 7: return launch_pdl(k_rk<Rp, Rs, PHYS, 1, 7>, grid, TPB, 0, s, a);
       default: return cudaErrorInvalidValue;
     }
   } else {
     switch (a.stage) {
-      case 1: k_rk<Rp, Rs, PHYS, 0, 1><<<grid, TPB, 0, s>>>(a); break;
-      case 2: k_rk<Rp, Rs, PHYS, 0, 2><<<grid, TPB, 0, s>>>(a); break;
-      case 3: k_rk<Rp, Rs, PHYS, 0, 3><<<grid, TPB, 0, s>>>(a); break;
-      case 4: k_rk<Rp, Rs, PHYS, 0, 4><<<grid, TPB, 0, s>>>(a); break;
-      case 5: k_rk<Rp, Rs, PHYS, 0, 5><<<grid, TPB, 0, s>>>(a); break;
-      case 6: k_rk<Rp, Rs, PHYS, 0, 6><<<grid, TPB, 0, s>>>(a); break;
-      case 7: k_rk<Rp, Rs, PHYS, 0, 7><<<grid, TPB, 0, s>>>(a); break;
+      case 1: return launch_pdl(k_rk<Rp, Rs, PHYS, 0, 1>, grid, TPB, 0, s, a);
+      case 2: return launch_pdl(k_rk<Rp, Rs, PHYS, 0, 2>, grid, TPB, 0, s, a);
+      case 3: return launch_pdl(k_rk<Rp, Rs, PHYS, 0, 3>, grid, TPB, 0, s, a);
+      case 4: return launch_pdl(k_rk<Rp, Rs, PHYS, 0, 4>, grid, TPB, 0, s, a);
+      case 5: return launch_pdl(k_rk<Rp, Rs, PHYS, 0, 5>, grid, TPB, 0, s, a);
+      case 6: return launch_pdl(k_rk<Rp, Rs, PHYS, 0, 6>, grid, TPB, 0, s, a);
+      case 7: return launch_pdl(k_rk<Rp, Rs, PHYS, 0, 7>, grid, TPB, 0, s, a);
       default: return cudaErrorInvalidValue;
     }
   }
-  return cudaGetLastError();
 }
 template <typename Rp, typename Rs>
 cudaError_t run_rk_phys(const RKArgs& a, int phys, int src, cudaStream_t s, int nblk) {
@@ -432,6 +432,7 @@ __device__ __forceinline__ void band_vector_force(int mode, const cx<double> (&v
 
 template <typename Ru>
 __global__ void __launch_bounds__(TPB) k_force_supply(ForceArgs a) {
+  pdl_wait();
   const Geo& g = a.g;
   const int ny = 2 * a.fy + 1, nz = a.fz + 1;
   const int box = (2 * a.fx + 1) * ny * nz;
@@ -526,6 +527,7 @@ struct PtrArr6 {
 
 template <typename Rp, int PHYS>
 __global__ void k_assemble_v(Geo g, PtrArr6 pa) {
+  pdl_wait();
   constexpr int NS = NState<PHYS>::v;
   const long long idx = (long long)blockIdx.x * TPB + threadIdx.x;
   if (idx >= g.S) return;
@@ -544,6 +546,7 @@ __global__ void k_assemble_v(Geo g, PtrArr6 pa) {
 }
 
 __global__ void k_sub_force_box(Geo g, int ncomp, const cx<double>* FB, int fx, int fy, int fz, PtrArr6 pa) {
+  pdl_wait();
   const int ny = 2 * fy + 1, nz = fz + 1;
   const int box = (2 * fx + 1) * ny * nz;
   const int p = blockIdx.x * TPB + threadIdx.x;
@@ -562,6 +565,7 @@ __global__ void k_sub_force_box(Geo g, int ncomp, const cx<double>* FB, int fx, 
 }
 
 __global__ void k_pressure(Geo g, PtrArr6 pa, cx<double>* PR) {
+  pdl_wait();
   const long long idx = (long long)blockIdx.x * TPB + threadIdx.x;
   if (idx >= g.S) return;
   int r1, r2, l3;
@@ -578,6 +582,7 @@ __global__ void k_pressure(Geo g, PtrArr6 pa, cx<double>* PR) {
 }
 
 __global__ void k_rhs_from_nlin(Geo g, int ns, PtrArr6 pa, const cx<double>* PR) {
+  pdl_wait();
   const long long idx = (long long)blockIdx.x * TPB + threadIdx.x;
   if (idx >= g.S) return;
   int r1, r2, l3;
@@ -596,6 +601,7 @@ __global__ void k_rhs_from_nlin(Geo g, int ns, PtrArr6 pa, const cx<double>* PR)
 // Add_force(T) for RB (add_force.cc:62-68) with Compute_force_RB: nlin1 -= fu theta,
 // T.nlin -= ft u1 (theta, u1 from the master state)
 __global__ void k_rb_sub_force(Geo g, PtrArr6 pa, const cx<double>* u1, const cx<double>* th, double fu, double ft) {
+  pdl_wait();
   const long long idx = (long long)blockIdx.x * TPB + threadIdx.x;
   if (idx >= g.S) return;
   pa.p[0][idx] = pa.p[0][idx] - fu * th[idx];
@@ -603,6 +609,7 @@ __global__ void k_rb_sub_force(Geo g, PtrArr6 pa, const cx<double>* u1, const cx
 }
 
 __global__ void k_sub_liquid_metal(Geo g, PtrArr6 nl, PtrArr6 u, double b0, double b1, double b2) {
+  pdl_wait();
   const long long idx = (long long)blockIdx.x * TPB + threadIdx.x;
   if (idx >= g.S) return;
   int r1, r2, l3;
@@ -615,6 +622,7 @@ __global__ void k_sub_liquid_metal(Geo g, PtrArr6 nl, PtrArr6 u, double b0, doub
 }
 
 __global__ void k_sub_coriolis(Geo g, PtrArr6 nl, PtrArr6 u, double o0, double o1, double o2) {
+  pdl_wait();
   const long long idx = (long long)blockIdx.x * TPB + threadIdx.x;
   if (idx >= g.S) return;
   const cx<double> v0 = u.p[0][idx], v1 = u.p[1][idx], v2 = u.p[2][idx];
@@ -649,6 +657,7 @@ __global__ void __launch_bounds__(TPB) k_cross_partials(Geo g, const cx<double>*
 }
 
 __global__ void __launch_bounds__(TPB) k_energy_partials(Geo g, PtrArr6 pa, int nf, double* part, int slot, int nslots) {
+  pdl_wait();
   double acc[2] = {0, 0};
   const long long stride = (long long)gridDim.x * TPB;
   for (long long idx = (long long)blockIdx.x * TPB + threadIdx.x; idx < g.S; idx += stride) {
@@ -682,26 +691,42 @@ __global__ void __launch_bounds__(TPB) k_energy_partials(Geo g, PtrArr6 pa, int 
   }
 }
 
-// one block per request r: sums its partials in a fixed order, then the dt rule of Get_dt
-// (compute_dt.cc:47-108); scal[8 r + 0..4] = dt, t, steps, non-finite flag, Tdt
-__global__ void __launch_bounds__(TPB) k_finalize(FinalizeArgs a) {
-  __shared__ double red[TPB];
-  const int r = blockIdx.x;
+// one block per request r: sums its partials (8 slots a block of the reducing kernel) in a fixed order,
+// then the dt rule of Get_dt (compute_dt.cc:47-108); scal[8 r + 0..4] = dt, t, steps, non-finite flag,
+// Tdt.  One launch in a chain of short ones: 128 blocks' partials are read at once, eight loads of a thread
+// in flight, so 888 blocks cost one round trip; slot after slot with 256 threads took 10 us a launch.
+constexpr int kFinThreads = 1024;
+__global__ void __launch_bounds__(kFinThreads) k_finalize(FinalizeArgs a) {
+  pdl_wait();
+  __shared__ double red[kFinThreads / 32][8];
+  const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int j = threadIdx.x & 7, b0 = threadIdx.x >> 3;
   const double* part = a.part + (long long)r * a.nblocks * a.nslots;
   double* out = a.out + (long long)r * a.nslots;
   double* scal = a.scal + (long long)r * 8;
-  for (int j = 0; j < a.nslots; ++j) {
-    double s = 0;
-    for (int b = threadIdx.x; b < a.nblocks; b += TPB) s += part[(long long)b * a.nslots + j];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = TPB / 2; o > 0; o >>= 1) {
-      if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-      __syncthreads();
+  double s = 0;
+  for (int base = 0; base < a.nblocks; base += kFinThreads) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int b = base + b0 + u * (kFinThreads / 8);
+      v[u] = (b < a.nblocks && j < a.nslots) ? part[(long long)b * a.nslots + j] : 0.0;
     }
-    if (threadIdx.x == 0) out[j] = red[0];
-    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += v[u];
   }
+  s += __shfl_down_sync(0xffffffffu, s, 16);
+  s += __shfl_down_sync(0xffffffffu, s, 8);
+  if (lane < 8) red[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0) return;
+  s = 0;
+#pragma unroll
+  for (int u = 0; u < kFinThreads / 128; ++u) s += red[(lane >> 3) * (kFinThreads / 128) + u][j];
+  s += __shfl_down_sync(0xffffffffu, s, 16);
+  s += __shfl_down_sync(0xffffffffu, s, 8);
+  if (lane < a.nslots) out[lane] = s;
+  __syncwarp();
   if (threadIdx.x != 0 || a.dt_mode == 0) return;
   const double Tdt = scal[4] > 0 ? scal[4] : a.Tdt;
   const double E = out[0] + (a.mhd ? out[2] : 0.0);
@@ -830,9 +855,7 @@ cudaError_t launch_rk(const RKArgs& a, int phys, int pprec, int sprec, int src, 
 }
 
 cudaError_t launch_force_supply(const ForceArgs& a, cudaStream_t s) {
-  if (a.uprec == 0) k_force_supply<double><<<1, TPB, 0, s>>>(a);
-  else k_force_supply<float><<<1, TPB, 0, s>>>(a);
-  return cudaGetLastError();
+  return launch_pdl(a.uprec == 0 ? k_force_supply<double> : k_force_supply<float>, 1, TPB, 0, s, a);
 }
 
 cudaError_t launch_assemble_nlin(const Geo& g, int phys, int pprec, const void* const* PX, cx<double>* const* NL, cudaStream_t s) {
@@ -844,9 +867,9 @@ cudaError_t launch_assemble_nlin(const Geo& g, int phys, int pprec, const void* 
   const int nb = nblk(g.S);
 #define TG_ASM(RP)                                                         \
   switch (phys) {                                                          \
-    case PH_FLUID: k_assemble_v<RP, PH_FLUID><<<nb, TPB, 0, s>>>(g, pa); break; \
-    case PH_MHD: k_assemble_v<RP, PH_MHD><<<nb, TPB, 0, s>>>(g, pa); break;     \
-    default: k_assemble_v<RP, PH_SCALAR><<<nb, TPB, 0, s>>>(g, pa); break;      \
+    case PH_FLUID: return launch_pdl(k_assemble_v<RP, PH_FLUID>, nb, TPB, 0, s, g, pa); \
+    case PH_MHD: return launch_pdl(k_assemble_v<RP, PH_MHD>, nb, TPB, 0, s, g, pa);     \
+    default: return launch_pdl(k_assemble_v<RP, PH_SCALAR>, nb, TPB, 0, s, g, pa);      \
   }
   if (pprec == 0) {
     TG_ASM(double)
@@ -854,38 +877,33 @@ cudaError_t launch_assemble_nlin(const Geo& g, int phys, int pprec, const void* 
     TG_ASM(float)
   }
 #undef TG_ASM
-  return cudaGetLastError();
 }
 
 cudaError_t launch_sub_force_box(const Geo& g, int ncomp, const cx<double>* FB, int fx, int fy, int fz, cx<double>* const* NL, cudaStream_t s) {
   PtrArr6 pa{};
   for (int c = 0; c < ncomp; ++c) pa.p[c] = NL[c];
   const int box = (2 * fx + 1) * (2 * fy + 1) * (fz + 1);
-  k_sub_force_box<<<(box + TPB - 1) / TPB, TPB, 0, s>>>(g, ncomp, FB, fx, fy, fz, pa);
-  return cudaGetLastError();
+  return launch_pdl(k_sub_force_box, (box + TPB - 1) / TPB, TPB, 0, s, g, ncomp, FB, fx, fy, fz, pa);
 }
 
 cudaError_t launch_pressure(const Geo& g, const cx<double>* const* NL, cx<double>* PR, cudaStream_t s) {
   PtrArr6 pa{};
   for (int c = 0; c < 3; ++c) pa.p[c] = const_cast<cx<double>*>(NL[c]);
-  k_pressure<<<nblk(g.S), TPB, 0, s>>>(g, pa, PR);
-  return cudaGetLastError();
+  return launch_pdl(k_pressure, nblk(g.S), TPB, 0, s, g, pa, PR);
 }
 
 cudaError_t launch_rhs_from_nlin(const Geo& g, int phys, cx<double>* const* NL, const cx<double>* PR, cudaStream_t s) {
   PtrArr6 pa{};
   const int ns = phys == PH_FLUID ? 3 : (phys == PH_MHD ? 6 : 4);
   for (int c = 0; c < ns; ++c) pa.p[c] = NL[c];
-  k_rhs_from_nlin<<<nblk(g.S), TPB, 0, s>>>(g, ns, pa, PR);
-  return cudaGetLastError();
+  return launch_pdl(k_rhs_from_nlin, nblk(g.S), TPB, 0, s, g, ns, pa, PR);
 }
 
 cudaError_t launch_rb_sub_force(const Geo& g, cx<double>* const* NL, const cx<double>* u1, const cx<double>* th,
                                 double fu, double ft, cudaStream_t s) {
   PtrArr6 pa{};
   for (int c = 0; c < 4; ++c) pa.p[c] = NL[c];
-  k_rb_sub_force<<<nblk(g.S), TPB, 0, s>>>(g, pa, u1, th, fu, ft);
-  return cudaGetLastError();
+  return launch_pdl(k_rb_sub_force, nblk(g.S), TPB, 0, s, g, pa, u1, th, fu, ft);
 }
 
 cudaError_t launch_sub_liquid_metal(const Geo& g, cx<double>* const* NL, const cx<double>* const* U, const double* b0,
@@ -895,8 +913,7 @@ cudaError_t launch_sub_liquid_metal(const Geo& g, cx<double>* const* NL, const c
     nl.p[c] = NL[c];
     u.p[c] = const_cast<cx<double>*>(U[c]);
   }
-  k_sub_liquid_metal<<<nblk(g.S), TPB, 0, s>>>(g, nl, u, b0[0], b0[1], b0[2]);
-  return cudaGetLastError();
+  return launch_pdl(k_sub_liquid_metal, nblk(g.S), TPB, 0, s, g, nl, u, b0[0], b0[1], b0[2]);
 }
 
 cudaError_t launch_sub_coriolis(const Geo& g, cx<double>* const* NL, const cx<double>* const* U, const double* om,
@@ -906,8 +923,7 @@ cudaError_t launch_sub_coriolis(const Geo& g, cx<double>* const* NL, const cx<do
     nl.p[c] = NL[c];
     u.p[c] = const_cast<cx<double>*>(U[c]);
   }
-  k_sub_coriolis<<<nblk(g.S), TPB, 0, s>>>(g, nl, u, om[0], om[1], om[2]);
-  return cudaGetLastError();
+  return launch_pdl(k_sub_coriolis, nblk(g.S), TPB, 0, s, g, nl, u, om[0], om[1], om[2]);
 }
 
 cudaError_t launch_cross_partials(const Geo& g, const cx<double>* A, const cx<double>* B, double* part, int slot,
@@ -923,13 +939,11 @@ cudaError_t launch_energy_partials(const Geo& g, const cx<double>* const* F, int
   for (int c = 0; c < nf; ++c) pa.p[c] = const_cast<cx<double>*>(F[c]);
   const int nb = nred(g.S);
   if (nblocks) *nblocks = nb;
-  k_energy_partials<<<dim3(nb, nact > 0 ? nact : 1), TPB, 0, s>>>(g, pa, nf, part, slot, nslots);
-  return cudaGetLastError();
+  return launch_pdl(k_energy_partials, dim3(nb, nact > 0 ? nact : 1), TPB, 0, s, g, pa, nf, part, slot, nslots);
 }
 
 cudaError_t launch_finalize(const FinalizeArgs& a, cudaStream_t s) {
-  k_finalize<<<a.nact > 0 ? a.nact : 1, TPB, 0, s>>>(a);
-  return cudaGetLastError();
+  return launch_pdl(k_finalize, a.nact > 0 ? a.nact : 1, kFinThreads, 0, s, a);
 }
 
 int shell_spectrum_blocks(const Geo& g) {
