@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "tg_ctx.h"
+#include "tg_xstage.h"
 
 using namespace tg;
 
@@ -139,10 +140,32 @@ int max_radius_inside(const tg_ctx* c) {
 // X-inverse, Y-inverse, fused z-pass (c2r, products, r2c), Y-forward, X-forward.
 // inputs: compact fields of precision inprec.  MHD: in[0..2] = U, in[3..5] = B, the x-pass
 // forms z+ = U + B (fields 0..2) and z- = U - B (fields 3..5).
+// the products of the trace-free form and their buffers
+struct TraceFree {
+  ProdPairs pp;
+  void *PP[8], *PY[8], *PX[8];
+  int kinds[8];
+  explicit TraceFree(const tg_ctx* c) {
+    for (int q = 0; q < c->nprod - 1; ++q) {
+      const int o = q < 2 ? q : q + 1;
+      pp.a[q] = c->pairs.a[o];
+      pp.b[q] = c->pairs.b[o];
+      if (q < 2) {
+        pp.c[q] = c->pairs.a[2];
+        pp.d[q] = c->pairs.b[2];
+      }
+      PP[q] = c->PP[o];
+      PY[q] = c->PY[o];
+      PX[q] = c->PX[o];
+      kinds[q] = c->xfwd_kind[o];
+    }
+  }
+};
+
 // trace_free: the products without the third square, which is taken from the first two
 // (u1u1 - u3u3, u2u2 - u3u3; z+- alike): five products instead of six, eight instead of nine.  Only for a
 // right-hand side that is projected: the velocity's term changes by a gradient.
-int run_pipeline(tg_ctx* c, const void* const* in, int inprec, bool trace_free) {
+int run_pipeline(tg_ctx* c, const void* const* in, int inprec, bool trace_free, bool have_x = false, bool leave_x = false) {
   const void* src[6];
   const void* src2[6] = {};
   int comb[6] = {0, 0, 0, 0, 0, 0};
@@ -155,26 +178,11 @@ int run_pipeline(tg_ctx* c, const void* const* in, int inprec, bool trace_free) 
       src[f] = in[f];
     }
   }
-  int rc = pipe_inverse_xy(c, c->nin, src, src2, comb, inprec, c->nstate, c->WX, c->WY);
+  int rc = pipe_inverse_xy(c, c->nin, src, src2, comb, inprec, c->nstate, c->WX, c->WY, have_x);
   if (rc) return rc;
   if (!trace_free) return pipe_products_forward(c, c->nin, c->WY, c->nprod, c->pairs, c->PP, c->PY, c->PX);
-  ProdPairs pp{};
-  void *PP[8], *PY[8], *PX[8];
-  int kinds[8];
-  for (int q = 0; q < c->nprod - 1; ++q) {
-    const int o = q < 2 ? q : q + 1;
-    pp.a[q] = c->pairs.a[o];
-    pp.b[q] = c->pairs.b[o];
-    if (q < 2) {
-      pp.c[q] = c->pairs.a[2];
-      pp.d[q] = c->pairs.b[2];
-    }
-    PP[q] = c->PP[o];
-    PY[q] = c->PY[o];
-    PX[q] = c->PX[o];
-    kinds[q] = c->xfwd_kind[o];
-  }
-  return pipe_products_forward(c, c->nin, c->WY, c->nprod - 1, pp, PP, PY, PX, kinds);
+  const TraceFree t(c);
+  return pipe_products_forward(c, c->nin, c->WY, c->nprod - 1, t.pp, t.PP, t.PY, t.PX, t.kinds, leave_x);
 }
 
 // whether a step's products are trace-free: always, but for FP64 MHD rows of N3 = 256, whose z-pass has
@@ -322,6 +330,7 @@ int scheme_stages(int scheme, int out[4]) {
 int run_stages(tg_ctx* c, int first, bool ring) {
   int st[4];
   const int ns_stages = scheme_stages(c->cfg.scheme, st);
+  bool have_x = false;  // WX holds the x-inverse of this stage's fields
   for (int si = first - 1; si < ns_stages; ++si) {
     const int stage = st[si];
     const void* in[6];
@@ -336,9 +345,36 @@ int run_stages(tg_ctx* c, int first, bool ring) {
     int rc = run_force(c, in, inprec);
     if (rc) return rc;
     const bool tf = step_trace_free(c);
-    rc = run_pipeline(c, in, inprec, tf);
+    const bool fuse = tf && !stage_is_final(stage) && xstage_fits(c->g, c->phys, c->tprec) && c->slab_W == 0;
+    rc = run_pipeline(c, in, inprec, tf, have_x, fuse);
     if (rc) return rc;
     RKArgs a = rk_args(c, stage);
+    have_x = false;
+    if (fuse) {
+      for (int i = 0; i < c->nstate; ++i) a.IN[i] = in[i];
+      a.inprec = (inprec == F64) ? 0 : 1;
+      XStageLaunch x;
+      x.phys = c->phys;
+      x.prec = c->tprec;
+      x.rk = a;
+      x.us_all = (c->coriolis || c->lm) ? 1 : 0;  // the next stage's force reads the whole field
+      x.tw = c->tw[c->N1];
+      x.wait_flag = c->wait_status;
+      x.wait_short = c->wait_short;
+      for (int q = 0; q < c->nprod - 1; ++q) x.src[q] = c->PY[q < 2 ? q : q + 1];  // as TraceFree
+      for (int i = 0; i < c->nin; ++i) x.dst[i] = c->WX[i];
+      {
+        const double ns = c->nstate, e = el_compact(c);
+        const double tot = (stage >= 2 && stage <= 3 ? 2 : (stage == 1 ? 1 : 0)) * ns * e * 16;
+        ProfScope pr(c, "x_stage", (c->nprod - 1 + ns) * el_xstage(c) * c->tsz + ns * e * 16 + tot);
+        TG_CK(launch_xstage(x, c->st, &have_x));
+      }
+      if (have_x) continue;
+      // refused (a tensor map that the driver does not take): the separate passes
+      const TraceFree t(c);
+      rc = pipe_forward_x(c, c->nprod - 1, t.PY, t.PX, t.kinds);
+      if (rc) return rc;
+    }
     if (tf) a.PX[2] = nullptr;
     for (int i = 0; i < c->nstate; ++i) a.IN[i] = in[i];
     a.inprec = (inprec == F64) ? 0 : 1;

@@ -177,13 +177,18 @@ double el_xstage(const tg_ctx* c);
 double el_ystage(const tg_ctx* c);
 
 // x- and y-inverse passes of nf compact fields (field f read as in[f] + comb[f] * in2[f]);
-// nread = number of distinct compact fields read (for the byte count)
+// nread = number of distinct compact fields read (for the byte count); have_x: WX holds the x-inverse
+// already, only the y pass runs
 int pipe_inverse_xy(tg_ctx* c, int nf, const void* const* in, const void* const* in2, const int* comb,
-                    int inprec, int nread, void* const* WX, void* const* WY);
+                    int inprec, int nread, void* const* WX, void* const* WY, bool have_x = false);
 // fused z-pass products (pairs pp of the nin inputs), then y- and x-forward passes into PX;
-// SCFT: product q takes the x transform xkinds[q] (0 cosine, 1 sine; default c->xfwd_kind)
+// SCFT: product q takes the x transform xkinds[q] (0 cosine, 1 sine; default c->xfwd_kind); leave_x: stop
+// after the y pass (PX is not written)
 int pipe_products_forward(tg_ctx* c, int nin, const void* const* WY, int nprod, const ProdPairs& pp,
-                          void* const* PP, void* const* PY, void* const* PX, const int* xkinds = nullptr);
+                          void* const* PP, void* const* PY, void* const* PX, const int* xkinds = nullptr,
+                          bool leave_x = false);
+// the x-forward pass alone
+int pipe_forward_x(tg_ctx* c, int nprod, void* const* PY, void* const* PX, const int* xkinds = nullptr);
 int dalloc_ctx(tg_ctx* c, void** p, size_t bytes);
 // a context holding B same-shape request slots (B = 1: tg_ctx_create); with slab_W > 0, rank
 // slab_r's share of a slab-sharded solve (B = 1)

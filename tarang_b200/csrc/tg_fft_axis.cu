@@ -20,6 +20,14 @@
 
 namespace tg {
 
+bool axis_tma_enabled() {
+  static const bool on = [] {
+    const char* e = std::getenv("TG_AXIS_TMA");
+    return !(e && e[0] == '0');
+  }();
+  return on;
+}
+
 namespace {
 
 // set by a TMA-staged block whose tile never arrived within the bounded wait
@@ -142,14 +150,6 @@ __global__ void __launch_bounds__(TmaW<Rw>::v * R1, AxisOcc<Rw, TmaW<Rw>::v * R1
     bulk_commit_group();
     bulk_wait_group_read0();
   }
-}
-
-bool axis_tma_enabled() {
-  static const bool on = [] {
-    const char* e = std::getenv("TG_AXIS_TMA");
-    return !(e && e[0] == '0');
-  }();
-  return on;
 }
 
 template <typename Ri, typename Ro, typename Rw, int R1, int R2, int DIR>

@@ -36,6 +36,8 @@ struct ZProdLaunch {
 };
 
 cudaError_t launch_axis(const AxisLaunch& l, cudaStream_t s);
+// false with TG_AXIS_TMA=0: the passes staged through registers instead of by TMA
+bool axis_tma_enabled();
 // 1 if a TMA-staged axis block gave up waiting for its tile (its output is not written), 0
 // otherwise, -1 if the flag cannot be read; clear resets it
 int axis_tma_timeout(bool clear);

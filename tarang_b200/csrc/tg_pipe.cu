@@ -40,10 +40,10 @@ double el_xstage(const tg_ctx* c) { return (double)c->N1 * c->g.nky * c->g.nkz; 
 double el_ystage(const tg_ctx* c) { return (double)c->N1 * c->N2 * c->g.nkz; }
 
 int pipe_inverse_xy(tg_ctx* c, int nf, const void* const* in, const void* const* in2, const int* comb,
-                    int inprec, int nread, void* const* WX, void* const* WY) {
+                    int inprec, int nread, void* const* WX, void* const* WY, bool have_x) {
   if (!c->pipeline_ok) return set_err(c, TG_ERR_UNSUPPORTED, "nonlinear term needs N3/2 a power of two in [4, 256]");
   const Geo& g = c->g;
-  {
+  if (!have_x) {
     AxisLaunch l;
     wait_args(c, l.a);
     l.L = c->N1;
@@ -116,7 +116,7 @@ int pipe_inverse_xy(tg_ctx* c, int nf, const void* const* in, const void* const*
 }
 
 int pipe_products_forward(tg_ctx* c, int nin, const void* const* WY, int nprod, const ProdPairs& pp,
-                          void* const* PP, void* const* PY, void* const* PX, const int* xkinds) {
+                          void* const* PP, void* const* PY, void* const* PX, const int* xkinds, bool leave_x) {
   if (!c->pipeline_ok) return set_err(c, TG_ERR_UNSUPPORTED, "nonlinear term needs N3/2 a power of two in [4, 256]");
   const Geo& g = c->g;
   {
@@ -168,6 +168,11 @@ int pipe_products_forward(tg_ctx* c, int nin, const void* const* WY, int nprod, 
     cudaError_t e = launch_axis(l, c->st);
     if (e != cudaSuccess) return cuda_err(c, e, "y forward");
   }
+  return leave_x ? TG_OK : pipe_forward_x(c, nprod, PY, PX, xkinds);
+}
+
+int pipe_forward_x(tg_ctx* c, int nprod, void* const* PY, void* const* PX, const int* xkinds) {
+  const Geo& g = c->g;
   {
     AxisLaunch l;
     wait_args(c, l.a);
