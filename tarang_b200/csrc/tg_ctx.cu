@@ -165,12 +165,13 @@ struct TraceFree {
 // trace_free: the products without the third square, which is taken from the first two
 // (u1u1 - u3u3, u2u2 - u3u3; z+- alike): five products instead of six, eight instead of nine.  Only for a
 // right-hand side that is projected: the velocity's term changes by a gradient.
-int run_pipeline(tg_ctx* c, const void* const* in, int inprec, bool trace_free, bool have_x = false, bool leave_x = false) {
+int run_pipeline(tg_ctx* c, const void* const* in, int inprec, bool trace_free, bool have_x = false, bool leave_x = false,
+                 bool have_z = false) {
   const void* src[6];
   const void* src2[6] = {};
   int comb[6] = {0, 0, 0, 0, 0, 0};
   for (int f = 0; f < c->nin; ++f) {
-    if (c->phys == TG_MHD) {
+    if (c->phys == TG_MHD && !have_z) {
       src[f] = in[f % 3];
       src2[f] = in[3 + f % 3];
       comb[f] = f < 3 ? +1 : -1;
@@ -331,6 +332,7 @@ int run_stages(tg_ctx* c, int first, bool ring) {
   int st[4];
   const int ns_stages = scheme_stages(c->cfg.scheme, st);
   bool have_x = false;  // WX holds the x-inverse of this stage's fields
+  bool have_z = false;  // MHD: the stage's fields in US are z+-
   for (int si = first - 1; si < ns_stages; ++si) {
     const int stage = st[si];
     const void* in[6];
@@ -346,7 +348,7 @@ int run_stages(tg_ctx* c, int first, bool ring) {
     if (rc) return rc;
     const bool tf = step_trace_free(c);
     const bool fuse = tf && !stage_is_final(stage) && xstage_fits(c->g, c->phys, c->tprec) && c->slab_W == 0;
-    rc = run_pipeline(c, in, inprec, tf, have_x, fuse);
+    rc = run_pipeline(c, in, inprec, tf, have_x, fuse, have_z);
     if (rc) return rc;
     RKArgs a = rk_args(c, stage);
     have_x = false;
@@ -376,6 +378,9 @@ int run_stages(tg_ctx* c, int first, bool ring) {
       if (rc) return rc;
     }
     if (tf) a.PX[2] = nullptr;
+    // MHD: the next stage's fields as the x-inverse takes them, unless a force reads them as U and B
+    have_z = c->phys == TG_MHD && !stage_is_final(stage) && c->force_on != 1 && !c->coriolis && !c->lm;
+    a.elsasser = have_z ? 1 : 0;
     for (int i = 0; i < c->nstate; ++i) a.IN[i] = in[i];
     a.inprec = (inprec == F64) ? 0 : 1;
     {

@@ -120,6 +120,7 @@ __global__ void __launch_bounds__(TPB, RKOcc<PHYS>::v) k_rk(RKArgs a) {
     }
     const int l1 = geo_l1(g, r1), l2 = amap_index(g.ay, r2);
     double eh = 0, e1 = 0;
+    cx<Rs> zu[3];  // MHD: the stage's U
 #pragma unroll
     for (int c = 0; c < NS; ++c) {
       if (c == 0 || nus[c] != nus[c - 1] || nuh[c] != nuh[c - 1]) {
@@ -130,7 +131,19 @@ __global__ void __launch_bounds__(TPB, RKOcc<PHYS>::v) k_rk(RKArgs a) {
       }
       const cx<double> rc = r[c];
       if constexpr (!FINAL) {
-        stc<Rs>(a.US[c], gi, stage_field<STAGE>(u0[c], rc, dt, eh));
+        const cx<Rs> us = cvt<Rs>(stage_field<STAGE>(u0[c], rc, dt, eh));
+        if constexpr (PHYS == PH_MHD) {
+          if (!a.elsasser) {
+            reinterpret_cast<cx<Rs>*>(a.US[c])[gi] = us;
+          } else if (c < 3) {
+            zu[c] = us;
+          } else {
+            reinterpret_cast<cx<Rs>*>(a.US[c - 3])[gi] = zu[c - 3] + us;
+            reinterpret_cast<cx<Rs>*>(a.US[c])[gi] = zu[c - 3] - us;
+          }
+        } else {
+          reinterpret_cast<cx<Rs>*>(a.US[c])[gi] = us;
+        }
         if constexpr (STAGE != 7) a.TOT[c][gi] = stage_total<STAGE>(STAGE == 1 ? mkc<double>(0, 0) : tot[c], rc, dt, eh, e1);
       } else {
         cx<double> u;

@@ -73,6 +73,7 @@ struct RKArgs {
   cx<double>* U0[6];       // FP64 master state
   cx<double>* TOT[6];      // FP64 RK accumulator
   void* US[6];             // stage fields (transform precision)
+  int elsasser;            // MHD: US takes z+ = U + B (0..2) and z- = U - B (3..5), the x-inverse's fields
   const void* PX[9];       // product spectra (compact)
   const cx<double>* RHS[6];// precomputed right-hand sides (SRC = 1)
   const cx<double>* FB;    // force box [nstate][box] or null
