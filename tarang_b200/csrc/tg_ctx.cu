@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "tg_ctx.h"
+#include "tg_hostcopy.h"
 #include "tg_xstage.h"
 
 using namespace tg;
@@ -567,6 +568,7 @@ void free_ctx(tg_ctx* c) {
   if (c->h_wait) cudaFreeHost(c->h_wait);
   if (c->own_stream && c->st) cudaStreamDestroy(c->st);
   delete c;
+  host_copy_release();
 }
 
 // Get_number_modes_in_shell_FOUR (four_basic.cc:48-105): inner <= |K| < outer, kz = 0 once,
@@ -637,10 +639,12 @@ int ctx_create_batch(const tg_config* cfg, int B, tg_ctx** out, int slab_W, int 
   const bool pipeline_ok = is_pow2(Mz) && Mz >= 4 && Mz <= 256;
 
   tg_ctx* c = new tg_ctx();
+  host_copy_retain();  // released by free_ctx
   c->cfg = *cfg;
   c->dev = cfg->device;
   cudaError_t e = cudaSetDevice(c->dev);
   if (e != cudaSuccess) {
+    host_copy_release();
     delete c;
     return TG_ERR_CUDA;
   }
@@ -648,6 +652,7 @@ int ctx_create_batch(const tg_config* cfg, int B, tg_ctx** out, int slab_W, int 
     c->st = (cudaStream_t)cfg->stream;
   } else {
     if (cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking) != cudaSuccess) {
+      host_copy_release();
       delete c;
       return TG_ERR_CUDA;
     }
@@ -1188,7 +1193,7 @@ int tg_field_upload(tg_ctx* c, int field, const double* host, size_t n) {
   if (field >= TG_WORK0 && field < TG_WORK0 + TG_NWORK) {
     int rc = ensure_dense(c, field);
     if (rc) return rc;
-    TG_CK(cudaMemcpyAsync(c->dense[field], host, sizeof(double) * n, cudaMemcpyHostToDevice, c->st));
+    TG_CK(host_copy(c->dense[field], host, sizeof(double) * n, true, c->dev, c->st));
     TG_SYNC(c, __func__);
     return TG_OK;
   }
@@ -1206,7 +1211,7 @@ int tg_field_upload(tg_ctx* c, int field, const double* host, size_t n) {
   else return set_err(c, TG_ERR_ARG, "upload: field not stored by this context");
   int rc = ensure_staging(c);
   if (rc) return rc;
-  TG_CK(cudaMemcpyAsync(c->staging, host, sizeof(double) * n, cudaMemcpyHostToDevice, c->st));
+  TG_CK(host_copy(c->staging, host, sizeof(double) * n, true, c->dev, c->st));
   TG_CK(launch_dense_to_compact(c->g, c->staging, target, 0, c->st));
   TG_SYNC(c, __func__);
   if (si >= 0) {
@@ -1223,7 +1228,7 @@ int tg_field_download(tg_ctx* c, int field, double* host, size_t n) {
   cudaSetDevice(c->dev);
   if (field >= TG_WORK0 && field < TG_WORK0 + TG_NWORK) {
     if (!c->dense[field]) return set_err(c, TG_ERR_STATE, "download: work field never written");
-    TG_CK(cudaMemcpyAsync(host, c->dense[field], sizeof(double) * n, cudaMemcpyDeviceToHost, c->st));
+    TG_CK(host_copy(host, c->dense[field], sizeof(double) * n, false, c->dev, c->st));
     TG_SYNC(c, __func__);
     return TG_OK;
   }
@@ -1288,7 +1293,7 @@ int tg_field_download(tg_ctx* c, int field, double* host, size_t n) {
   int rc = ensure_staging(c);
   if (rc) return rc;
   TG_CK(launch_compact_to_dense(c->g, src, sp, c->staging, c->st));
-  TG_CK(cudaMemcpyAsync(host, c->staging, sizeof(double) * n, cudaMemcpyDeviceToHost, c->st));
+  TG_CK(host_copy(host, c->staging, sizeof(double) * n, false, c->dev, c->st));
   TG_SYNC(c, __func__);
   return TG_OK;
 }

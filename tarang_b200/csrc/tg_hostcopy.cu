@@ -1,0 +1,227 @@
+// The driver copies pageable memory with one thread through its own page-locked buffer: 19 to 20 GB/s either
+// way on the host measured, where the bus takes 52 and four threads copy 47 GB/s in memory.  Here a few
+// threads take the pieces of a copy in turn; each brings a piece between the caller's memory and a
+// page-locked slot of its own and queues the transfer of the slot on the stream, so that the transfers and
+// the copies of other pieces overlap.  One copy runs at a time; a second caller meanwhile, or a host that
+// gives no threads or page-locked memory, gets the driver's copy.
+// Measured (B200 host, 16 cores, 17 MB field): MEASURED_HOSTCOPY
+#include "tg_hostcopy.h"
+
+#include <algorithm>
+#include <atomic>
+#include <condition_variable>
+#include <cstring>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+namespace tg {
+
+namespace {
+
+constexpr size_t kPiece = 1 << 20;
+constexpr size_t kMinBytes = 4 * kPiece;  // shorter copies do not fill the threads
+constexpr int kMaxThreads = 4;
+constexpr int kSlots = 2;  // per thread: one in transfer, one being copied
+
+struct Job {
+  char* host = nullptr;
+  char* dev = nullptr;
+  size_t bytes = 0;
+  bool to_device = false;
+  int device = 0;
+  cudaStream_t s = nullptr;
+};
+
+class Copier {
+ public:
+  // threads and slots; false when the host does not give them
+  bool start() {
+    const unsigned hw = std::thread::hardware_concurrency();
+    const int n = (int)std::min<unsigned>(kMaxThreads, hw / 2);
+    if (n < 2) return false;
+    if (cudaHostAlloc((void**)&pin_, (size_t)n * kSlots * kPiece, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      pin_ = nullptr;
+      return false;
+    }
+    try {
+      for (int i = 0; i < n; ++i) threads_.emplace_back([this, i] { loop(i); });
+    } catch (...) {
+      stop();
+      return false;
+    }
+    return true;
+  }
+  void stop() {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      quit_ = true;
+    }
+    cv_.notify_all();
+    for (auto& t : threads_) t.join();
+    threads_.clear();
+    if (pin_) cudaFreeHost(pin_);
+    pin_ = nullptr;
+  }
+  cudaError_t run(const Job& j) {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      job_ = j;
+      err_ = cudaSuccess;
+      next_.store(0);
+      left_ = (int)threads_.size();
+      ++turn_;
+    }
+    cv_.notify_all();
+    std::unique_lock<std::mutex> lk(mu_);
+    done_.wait(lk, [this] { return left_ == 0; });
+    return err_;
+  }
+
+ private:
+  void loop(int id) {
+    unsigned seen = 0;
+    for (;;) {
+      Job j;
+      {
+        std::unique_lock<std::mutex> lk(mu_);
+        cv_.wait(lk, [&] { return quit_ || turn_ != seen; });
+        if (quit_) return;
+        seen = turn_;
+        j = job_;
+      }
+      const cudaError_t e = work(j, pin_ + (size_t)id * kSlots * kPiece);
+      {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (e != cudaSuccess && err_ == cudaSuccess) err_ = e;
+        if (--left_ == 0) done_.notify_one();
+      }
+    }
+  }
+  // this thread's pieces of a job: the slots in turn, a slot's transfer ended before it is used again
+  cudaError_t work(const Job& j, char* slot0) {
+    cudaError_t e = cudaSetDevice(j.device);
+    cudaEvent_t ev[kSlots] = {};
+    for (int i = 0; i < kSlots && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
+    const size_t n = (j.bytes + kPiece - 1) / kPiece;
+    size_t held[kSlots];  // D2H: the piece whose transfer into the slot is under way
+    bool busy[kSlots] = {};
+    auto finish = [&](int i) {
+      if (!busy[i]) return cudaSuccess;
+      busy[i] = false;
+      const cudaError_t r = cudaEventSynchronize(ev[i]);
+      if (r == cudaSuccess && !j.to_device) {
+        const size_t o = held[i] * kPiece;
+        std::memcpy(j.host + o, slot0 + (size_t)i * kPiece, std::min(kPiece, j.bytes - o));
+      }
+      return r;
+    };
+    int i = 0;
+    while (e == cudaSuccess) {
+      const size_t p = next_.fetch_add(1);
+      if (p >= n) break;
+      e = finish(i);
+      if (e != cudaSuccess) break;
+      char* slot = slot0 + (size_t)i * kPiece;
+      const size_t o = p * kPiece, len = std::min(kPiece, j.bytes - o);
+      if (j.to_device) {
+        std::memcpy(slot, j.host + o, len);
+        e = cudaMemcpyAsync(j.dev + o, slot, len, cudaMemcpyHostToDevice, j.s);
+      } else {
+        e = cudaMemcpyAsync(slot, j.dev + o, len, cudaMemcpyDeviceToHost, j.s);
+      }
+      if (e == cudaSuccess) e = cudaEventRecord(ev[i], j.s);
+      held[i] = p;
+      busy[i] = e == cudaSuccess;
+      i = (i + 1) % kSlots;
+    }
+    for (int k = 0; k < kSlots; ++k, i = (i + 1) % kSlots) {
+      const cudaError_t r = finish(i);
+      if (e == cudaSuccess) e = r;
+    }
+    for (int k = 0; k < kSlots; ++k)
+      if (ev[k]) cudaEventDestroy(ev[k]);
+    return e;
+  }
+
+  std::vector<std::thread> threads_;
+  char* pin_ = nullptr;
+  std::mutex mu_;
+  std::condition_variable cv_, done_;
+  Job job_;
+  std::atomic<size_t> next_{0};
+  int left_ = 0;
+  unsigned turn_ = 0;
+  bool quit_ = false;
+  cudaError_t err_ = cudaSuccess;
+};
+
+std::mutex g_busy;         // one copy at a time; also guards the two below
+Copier* g_copier = nullptr;
+bool g_refused = false;    // the host gave no threads or slots: not asked again until the owners have left
+std::mutex g_owners_mu;
+int g_owners = 0;
+
+}  // namespace
+
+void host_copy_retain() {
+  std::lock_guard<std::mutex> lk(g_owners_mu);
+  ++g_owners;
+}
+
+void host_copy_release() {
+  std::lock_guard<std::mutex> lk(g_owners_mu);
+  if (--g_owners > 0) return;
+  std::lock_guard<std::mutex> b(g_busy);
+  if (g_copier) {
+    g_copier->stop();
+    delete g_copier;
+    g_copier = nullptr;
+  }
+  g_refused = false;
+}
+
+cudaError_t host_copy(void* dst, const void* src, size_t bytes, bool to_device, int device, cudaStream_t s) {
+  const void* host = to_device ? src : dst;
+  bool staged = bytes >= kMinBytes;
+  if (staged) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+      cudaGetLastError();
+      staged = false;
+    } else {
+      staged = at.type == cudaMemoryTypeUnregistered;
+    }
+  }
+  if (staged) {
+    std::unique_lock<std::mutex> lk(g_busy, std::try_to_lock);
+    if (lk.owns_lock()) {
+      if (!g_copier && !g_refused) {
+        try {
+          g_copier = new Copier;
+        } catch (...) {
+        }
+        if (g_copier && !g_copier->start()) {
+          delete g_copier;
+          g_copier = nullptr;
+        }
+        g_refused = g_copier == nullptr;
+      }
+      if (g_copier) {
+        Job j;
+        j.host = static_cast<char*>(const_cast<void*>(host));
+        j.dev = static_cast<char*>(to_device ? dst : const_cast<void*>(src));
+        j.bytes = bytes;
+        j.to_device = to_device;
+        j.device = device;
+        j.s = s;
+        return g_copier->run(j);
+      }
+    }
+  }
+  cudaError_t e = cudaMemcpyAsync(dst, src, bytes, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, s);
+  return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+
+}  // namespace tg

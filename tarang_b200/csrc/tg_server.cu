@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "tg_ctx.h"
+#include "tg_hostcopy.h"
 
 using namespace tg;
 
@@ -574,11 +575,13 @@ int tg_server_create(const tg_server_config* cfg, tg_server** out) {
   if (cfg->hbm_budget_bytes == 0 || cfg->max_batch < 1) return TG_ERR_ARG;
   if (cudaSetDevice(cfg->device) != cudaSuccess) return TG_ERR_CUDA;
   tg_server* s = new tg_server();
+  host_copy_retain();
   s->cfg = *cfg;
   s->dev = cfg->device;
   if (cudaStreamCreateWithFlags(&s->aux, cudaStreamNonBlocking) != cudaSuccess) {
     cudaGetLastError();
     delete s;
+    host_copy_release();
     return TG_ERR_CUDA;
   }
   // the kept results' pool keeps freed memory mapped (a pool that hands memory back at every
@@ -591,6 +594,7 @@ int tg_server_create(const tg_server_config* cfg, tg_server** out) {
     cudaGetLastError();
     cudaStreamDestroy(s->aux);
     delete s;
+    host_copy_release();
     return TG_ERR_CUDA;
   }
   unsigned long long keep = ~0ull;
@@ -619,6 +623,7 @@ int tg_server_destroy(tg_server* s) {
     if (kv.second.init_pin) cudaFreeHost(kv.second.init_pin);
   s->pinned.clear();
   delete s;
+  host_copy_release();
   return TG_OK;
 }
 
@@ -793,8 +798,7 @@ int tg_server_result(tg_server* s, long long id, double* host, size_t n) {
   // on the server's own non-blocking stream, after the result's copies, so that the batches'
   // streams go on
   cudaError_t e = r.result_ev ? cudaStreamWaitEvent(s->aux, r.result_ev, 0) : cudaSuccess;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(host, r.result, sizeof(double) * n, cudaMemcpyDeviceToHost, s->aux);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s->aux);
+  if (e == cudaSuccess) e = host_copy(host, r.result, sizeof(double) * n, false, s->dev, s->aux);
   if (e != cudaSuccess) {
     s->err = std::string("result download: ") + cudaGetErrorString(e);
     return TG_ERR_CUDA;
