@@ -4,7 +4,7 @@
 // page-locked slot of its own and queues the transfer of the slot on the stream, so that the transfers and
 // the copies of other pieces overlap.  One copy runs at a time; a second caller meanwhile, or a host that
 // gives no threads or page-locked memory, gets the driver's copy.
-// Measured (B200 host, 16 cores, 17 MB field): MEASURED_HOSTCOPY
+// Measured (B200 host, 16 cores, 17 MB field): upload 0.885 -> 0.528 ms, download 0.851 -> 0.518 (page-locked 0.33 and 0.32).
 #include "tg_hostcopy.h"
 
 #include <algorithm>
