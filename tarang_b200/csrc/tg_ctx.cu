@@ -180,11 +180,19 @@ int run_pipeline(tg_ctx* c, const void* const* in, int inprec, bool trace_free, 
       src[f] = in[f];
     }
   }
-  int rc = pipe_inverse_xy(c, c->nin, src, src2, comb, inprec, c->nstate, c->WX, c->WY, have_x);
-  if (rc) return rc;
-  if (!trace_free) return pipe_products_forward(c, c->nin, c->WY, c->nprod, c->pairs, c->PP, c->PY, c->PX);
   const TraceFree t(c);
-  return pipe_products_forward(c, c->nin, c->WY, c->nprod - 1, t.pp, t.PP, t.PY, t.PX, t.kinds, leave_x);
+  const int nprod = trace_free ? c->nprod - 1 : c->nprod;
+  int rc = TG_OK;
+  if (plane_taken(c, nprod)) {
+    rc = have_x ? TG_OK : pipe_inverse_xy(c, c->nin, src, src2, comb, inprec, c->nstate, c->WX, c->WY, false, true);
+    if (!rc) rc = pipe_plane(c, c->nin, c->WX, nprod, trace_free ? t.pp : c->pairs, trace_free ? t.PY : c->PY);
+    if (rc || leave_x) return rc;
+    return trace_free ? pipe_forward_x(c, nprod, t.PY, t.PX, t.kinds) : pipe_forward_x(c, nprod, c->PY, c->PX);
+  }
+  rc = pipe_inverse_xy(c, c->nin, src, src2, comb, inprec, c->nstate, c->WX, c->WY, have_x);
+  if (rc) return rc;
+  if (!trace_free) return pipe_products_forward(c, c->nin, c->WY, nprod, c->pairs, c->PP, c->PY, c->PX);
+  return pipe_products_forward(c, c->nin, c->WY, nprod, t.pp, t.PP, t.PY, t.PX, t.kinds, leave_x);
 }
 
 // whether a step's products are trace-free: always, but for FP64 MHD rows of N3 = 256, whose z-pass has

@@ -178,15 +178,19 @@ double el_ystage(const tg_ctx* c);
 
 // x- and y-inverse passes of nf compact fields (field f read as in[f] + comb[f] * in2[f]);
 // nread = number of distinct compact fields read (for the byte count); have_x: WX holds the x-inverse
-// already, only the y pass runs
+// already, only the y pass runs; leave_y: stop after the x pass (WY is not written)
 int pipe_inverse_xy(tg_ctx* c, int nf, const void* const* in, const void* const* in2, const int* comb,
-                    int inprec, int nread, void* const* WX, void* const* WY, bool have_x = false);
+                    int inprec, int nread, void* const* WX, void* const* WY, bool have_x = false,
+                    bool leave_y = false);
 // fused z-pass products (pairs pp of the nin inputs), then y- and x-forward passes into PX;
 // SCFT: product q takes the x transform xkinds[q] (0 cosine, 1 sine; default c->xfwd_kind); leave_x: stop
 // after the y pass (PX is not written)
 int pipe_products_forward(tg_ctx* c, int nin, const void* const* WY, int nprod, const ProdPairs& pp,
                           void* const* PP, void* const* PY, void* const* PX, const int* xkinds = nullptr,
                           bool leave_x = false);
+// y-inverse, z-pass products and y-forward of WX into PY in one kernel, where the plane fits it
+bool plane_taken(const tg_ctx* c, int nprod);
+int pipe_plane(tg_ctx* c, int nin, void* const* WX, int nprod, const ProdPairs& pp, void* const* PY);
 // the x-forward pass alone
 int pipe_forward_x(tg_ctx* c, int nprod, void* const* PY, void* const* PX, const int* xkinds = nullptr);
 int dalloc_ctx(tg_ctx* c, void** p, size_t bytes);

@@ -1,16 +1,31 @@
 // The pass sequence of a nonlinear product term on the compact layout:
 //   x-inverse -> y-inverse (pipe_inverse_xy) and
-//   fused z-pass (c2r, pointwise products, r2c) -> y-forward -> x-forward (pipe_products_forward).
+//   fused z-pass (c2r, pointwise products, r2c) -> y-forward -> x-forward (pipe_products_forward);
+// where a y-z plane fits in shared memory: x-inverse -> pipe_plane -> x-forward (pipe_forward_x).
 // Used by the time step (IncVF::Compute_nlin) and by the energy-transfer diagnostics
 // (IncVF::EnergyTr_Compute_nlin).
 #include <algorithm>
 
 #include "tg_ctx.h"
+#include "tg_plane.h"
 
 namespace tg {
 
 namespace {
 AxisMap full_map(int L) { return AxisMap{L, L, 0}; }
+
+void plane_shape(const tg_ctx* c, int nprod, PlaneLaunch& l) {
+  l.N2 = c->N2;
+  l.M = c->Mz;
+  l.prec = c->tprec;
+  l.nplanes = (long long)c->nact * c->N1;
+  l.a.ay = c->g.ay;
+  l.a.nky = c->g.nky;
+  l.a.kzp = c->g.kzp;
+  l.a.nkz = c->g.nkz;
+  l.a.nin = c->nin;
+  l.a.nprod = nprod;
+}
 }  // namespace
 
 cudaEvent_t prof_event(tg_ctx* c) {
@@ -40,7 +55,7 @@ double el_xstage(const tg_ctx* c) { return (double)c->N1 * c->g.nky * c->g.nkz; 
 double el_ystage(const tg_ctx* c) { return (double)c->N1 * c->N2 * c->g.nkz; }
 
 int pipe_inverse_xy(tg_ctx* c, int nf, const void* const* in, const void* const* in2, const int* comb,
-                    int inprec, int nread, void* const* WX, void* const* WY, bool have_x) {
+                    int inprec, int nread, void* const* WX, void* const* WY, bool have_x, bool leave_y) {
   if (!c->pipeline_ok) return set_err(c, TG_ERR_UNSUPPORTED, "nonlinear term needs N3/2 a power of two in [4, 256]");
   const Geo& g = c->g;
   if (!have_x) {
@@ -87,6 +102,7 @@ int pipe_inverse_xy(tg_ctx* c, int nf, const void* const* in, const void* const*
     }
     if (e != cudaSuccess) return cuda_err(c, e, "x inverse");
   }
+  if (leave_y) return TG_OK;
   {
     AxisLaunch l;
     wait_args(c, l.a);
@@ -169,6 +185,26 @@ int pipe_products_forward(tg_ctx* c, int nin, const void* const* WY, int nprod, 
     if (e != cudaSuccess) return cuda_err(c, e, "y forward");
   }
   return leave_x ? TG_OK : pipe_forward_x(c, nprod, PY, PX, xkinds);
+}
+
+bool plane_taken(const tg_ctx* c, int nprod) {
+  PlaneLaunch l;
+  plane_shape(c, nprod, l);
+  return c->pipeline_ok && c->slab_W == 0 && plane_fits(l, c->N1);
+}
+
+int pipe_plane(tg_ctx* c, int nin, void* const* WX, int nprod, const ProdPairs& pp, void* const* PY) {
+  PlaneLaunch l;
+  plane_shape(c, nprod, l);
+  l.a.scale = 1.0 / ((double)c->N1 * c->N2 * c->N3);
+  l.a.twy = c->tw[c->N2];
+  l.a.twN = c->tw[c->N3];
+  for (int f = 0; f < nin; ++f) l.ps.src[f] = WX[f];
+  for (int q = 0; q < nprod; ++q) l.ps.dst[q] = PY[q];
+  l.pp = pp;
+  ProfScope pr(c, "yz_plane", (nin + nprod) * el_xstage(c) * c->tsz);
+  const cudaError_t e = launch_plane(l, c->st);
+  return e == cudaSuccess ? TG_OK : cuda_err(c, e, "y-z plane");
 }
 
 int pipe_forward_x(tg_ctx* c, int nprod, void* const* PY, void* const* PX, const int* xkinds) {
