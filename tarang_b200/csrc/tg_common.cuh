@@ -97,7 +97,7 @@ __device__ __forceinline__ void warp_bin_add(double* row, int bin, double v, boo
 // The wait returns when the kernels before have ended and their memory operations are visible, and
 // every thread of every block passes through it, so a kernel never ends before its predecessor and the
 // order of the stream holds through any number of them.
-// Measured (B200, step graphs, with and without): 32^3 FP32-mixed fluid 66.5 / 74.0 us, 64^3 FP64 102.0 /
+// Measured (B200, step graphs of one kernel a pass, with and without): 32^3 FP32-mixed fluid 66.5 / 74.0 us, 64^3 FP64 102.0 /
 // 110.7, 128^3 FP32-mixed 280.6 / 283.1, 256^3 unchanged.  No kernel lets its successor in early
 // (griddepcontrol.launch_dependents at its start): that took 270.6 us at 128^3 FP32-mixed, but 113.2 at
 // 64^3 and 1817 against 1685 us at 256^3 FP32-mixed, 3610 against 3205 for MHD there (waiting blocks

@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(kFinThreads) k_finalize(FinalizeArgs a) {
 
 // Shell sums of the fields' energies (and the mode counts) in a fixed order: per warp a row of
 // bins (warp_bin_add: the lanes of a shell in lane order), the block's rows in warp order into
-// part[block], then k_bins_accumulate adds the blocks in block order to ek / cnt -- the same bits
+// part[block], then k_bins_accumulate adds the blocks in a fixed order to ek / cnt -- the same bits
 // on every run
 __global__ void __launch_bounds__(TPB) k_shell_spectrum(Geo g, PtrArr6 pa, int nf, double n_pow, double* part,
                                                         int nbins) {

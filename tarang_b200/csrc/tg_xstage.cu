@@ -311,7 +311,7 @@ cudaError_t run_xstage_p(const XStageLaunch& l, cudaStream_t s, bool* used) {
 // The lines: a grid whose tiles fit one wave of two blocks an SM is a latency chain, where three launches
 // in one win whatever the kernel's own rate.  A larger grid is taken where the fused kernel, at 20 warps an
 // SM, still beats the three passes at 24 to 48: FP64 fluid with N1 = 256 or 64.  Steps measured (fused /
-// separate, us): 32^3 FP32 fluid 59.6 / 66.5, MHD 67.8 / 76.0; 64^3 FP64 fluid 94.5 / 102.0, scalar 124 / 135,
+// separate, us, the y and z passes one by one): 32^3 FP32 fluid 59.6 / 66.5, MHD 67.8 / 76.0; 64^3 FP64 fluid 94.5 / 102.0, scalar 124 / 135,
 // FP32 MHD 98 / 107; 256 x 64 x 64 FP64 256 / 282; 256^3 FP64 2806 / 3000; 64 x 256 x 256 FP64 806 / 829; and
 // against it 64 x 256 x 256 FP32 500 / 475, MHD 901 / 846, 128^3 FP64 463 / 448, 256^3 FP32 1686 / 1647.
 // Looks at one request's geometry only, so a batched request takes the path of a lone one.
