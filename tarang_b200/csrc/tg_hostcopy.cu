@@ -184,7 +184,9 @@ void host_copy_release() {
 
 cudaError_t host_copy(void* dst, const void* src, size_t bytes, bool to_device, int device, cudaStream_t s) {
   const void* host = to_device ? src : dst;
-  bool staged = bytes >= kMinBytes;
+  // the per-thread handle names another stream in each of the threads, which would order nothing behind
+  // the caller's work: the driver's copy, from the calling thread
+  bool staged = bytes >= kMinBytes && s != cudaStreamPerThread;
   if (staged) {
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
