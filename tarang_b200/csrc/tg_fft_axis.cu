@@ -370,9 +370,14 @@ cudaError_t run_r2r_fold(const AxisLaunch& l, const R2RArgs& r, cudaStream_t s, 
              : run_r2r_fold_rt<Ri, 11, false>(l, r, ntile, steps, vec, s);
 }
 
+// shared memory of k_axis_r2r_dmma: the ring of input stages and the block's coefficients
+size_t dmma_smem(int mt, int nst) {
+  return sizeof(double) * ((size_t)kDmStages * kDmStageD + (size_t)nst * (kDmPairs / 4) * 2 * mt * 32);
+}
+
 template <int MT, bool FWD>
 cudaError_t run_r2r_dmma_mt(const AxisLaunch& l, const R2RArgs& r, int nrb, int nst, cudaStream_t s) {
-  const size_t smem = sizeof(double) * ((size_t)kDmStages * kDmStageD + (size_t)nst * (kDmPairs / 4) * 2 * MT * 32);
+  const size_t smem = dmma_smem(MT, nst);
   auto kern = k_axis_r2r_dmma<MT, FWD>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -385,8 +390,11 @@ cudaError_t run_r2r_dmma_mt(const AxisLaunch& l, const R2RArgs& r, int nrb, int 
 }
 
 // FP64: the folded product on the matrix instructions.  Row tiles of 8 MT pairs with MT the smaller
-// of two values that needs no more row blocks than the larger (N1 = 129, 128: 6 forward, 9 inverse in
-// one block; N1 = 65: 3 and 5).
+// of the two larger values if that needs no more row blocks (N1 = 129, 128: 6 forward, 9 inverse in
+// one block; N1 = 65: 3 and 5), and the next smaller one while the coefficients of a block's rows do
+// not fit beside the ring: MT = 2 fits every N1 of launch_r2r (196 KB at 1024).  Measured convection
+// steps against the register-tiled product of the full matrix (us): N1 x 16 x 32 with N1 = 417 309 / 869,
+// 513 451 / 1354; all modes stored 404 639 / 1659, 600 1320 / 4868.
 cudaError_t run_r2r_dmma(const AxisLaunch& l, const R2RArgs& r, cudaStream_t s, bool* used) {
   *used = false;
   bool fwd;
@@ -396,14 +404,16 @@ cudaError_t run_r2r_dmma(const AxisLaunch& l, const R2RArgs& r, cudaStream_t s, 
     if (((reinterpret_cast<uintptr_t>(l.ps.src[f]) | reinterpret_cast<uintptr_t>(l.ps.dst[f])) & 15) != 0) return cudaSuccess;
   const int pairs = fwd ? (nout + 1) / 2 : (N + 1) / 2, mts = (pairs + 7) / 8;
   const int nst = ((fwd ? (N + 1) / 2 : (nin + 1) / 2) + kDmPairs - 1) / kDmPairs;
-  const int big = fwd ? 6 : 9, small = fwd ? 3 : 5;
-  const int mt = (mts + small - 1) / small <= (mts + big - 1) / big ? small : big;
-  const int nrb = (mts + mt - 1) / mt;
-  const size_t smem = sizeof(double) * ((size_t)kDmStages * kDmStageD + (size_t)nst * (kDmPairs / 4) * 2 * mt * 32);
-  if (smem > 227 * 1024 || (long long)l.nfields * nrb > 65535) return cudaSuccess;
+  const int tile[3] = {fwd ? 6 : 9, fwd ? 3 : 5, 2};
+  int t = (mts + tile[1] - 1) / tile[1] <= (mts + tile[0] - 1) / tile[0] ? 1 : 0;
+  while (t < 3 && dmma_smem(tile[t], nst) > 227 * 1024) ++t;
+  if (t == 3) return cudaSuccess;
+  const int nrb = (mts + tile[t] - 1) / tile[t];
+  if ((long long)l.nfields * nrb > 65535) return cudaSuccess;
   *used = true;
-  if (fwd) return mt == 3 ? run_r2r_dmma_mt<3, true>(l, r, nrb, nst, s) : run_r2r_dmma_mt<6, true>(l, r, nrb, nst, s);
-  return mt == 5 ? run_r2r_dmma_mt<5, false>(l, r, nrb, nst, s) : run_r2r_dmma_mt<9, false>(l, r, nrb, nst, s);
+  if (t == 2) return fwd ? run_r2r_dmma_mt<2, true>(l, r, nrb, nst, s) : run_r2r_dmma_mt<2, false>(l, r, nrb, nst, s);
+  if (fwd) return t == 1 ? run_r2r_dmma_mt<3, true>(l, r, nrb, nst, s) : run_r2r_dmma_mt<6, true>(l, r, nrb, nst, s);
+  return t == 1 ? run_r2r_dmma_mt<5, false>(l, r, nrb, nst, s) : run_r2r_dmma_mt<9, false>(l, r, nrb, nst, s);
 }
 
 // FP32 forms: the x-inverse contraction on the tensor cores (k_axis_r2r_tc, 3xTF32) when a field of
