@@ -131,7 +131,10 @@ class Copier {
       } else {
         e = cudaMemcpyAsync(slot, j.dev + o, len, cudaMemcpyDeviceToHost, j.s);
       }
-      if (e == cudaSuccess) e = cudaEventRecord(ev[i], j.s);
+      if (e == cudaSuccess) {
+        e = cudaEventRecord(ev[i], j.s);
+        if (e != cudaSuccess) cudaStreamSynchronize(j.s);  // the slot's transfer is queued all the same
+      }
       held[i] = p;
       busy[i] = e == cudaSuccess;
       i = (i + 1) % kSlots;

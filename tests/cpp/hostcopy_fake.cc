@@ -31,12 +31,18 @@ std::mutex mu;
 std::map<Key, Queue> queues;
 std::thread::id caller;
 int staged_copies = 0;     // transfers queued by a thread that is not the caller
+int records = 0, fail_record = -1;
 
 Queue* queue_of(cudaStream_t s) {
   return &queues[Key(s, s == cudaStreamPerThread ? std::this_thread::get_id() : std::thread::id())];
 }
 void run(Queue* q, size_t upto) {
   for (; q->done < upto; ++q->done) q->ops[q->done]();
+}
+size_t in_flight() {
+  size_t n = 0;
+  for (auto& kv : queues) n += kv.second.ops.size() - kv.second.done;
+  return n;
 }
 
 }  // namespace
@@ -67,6 +73,7 @@ cudaError_t cudaEventDestroy(cudaEvent_t e) {
 }
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
   std::lock_guard<std::mutex> lk(mu);
+  if (fail_record >= 0 && records++ >= fail_record) return cudaErrorUnknown;
   Event* ev = reinterpret_cast<Event*>(e);
   ev->q = queue_of(s);
   ev->upto = ev->q->ops.size();
@@ -134,6 +141,18 @@ int main(int argc, char** argv) {
     CHECK(dev == want);
     CHECK(seen == std::vector<unsigned char>(n, 0));
     CHECK(s == cudaStreamPerThread || staged_copies > 0);
+  } else if (!std::strcmp(what, "record_fails")) {
+    // events that cannot be recorded: the call fails, and no transfer is left in flight on the slots
+    for (int at : {0, 2, 5}) {
+      records = 0;
+      fail_record = at;
+      CHECK(tg::host_copy(dev.data(), want.data(), n, true, 0, s) != cudaSuccess);
+      CHECK(in_flight() == 0);
+      fail_record = -1;
+      CHECK(tg::host_copy(dev.data(), want.data(), n, true, 0, s) == cudaSuccess);
+      CHECK(dev == want);
+    }
+    CHECK(staged_copies > 0);
   } else {
     return 2;
   }

@@ -1,5 +1,6 @@
 """The threaded host copies against a fake CUDA runtime (tests/cpp/hostcopy_fake.cc): streams that run
-nothing until they are waited for, and a per-thread stream handle that names another queue in every thread."""
+nothing until they are waited for, a per-thread stream handle that names another queue in every thread, and an
+event that cannot be recorded."""
 
 import os
 import shutil
@@ -25,4 +26,9 @@ def program(tmp_path_factory):
 @pytest.mark.parametrize("scenario", ["download", "upload", "download_per_thread", "upload_per_thread"])
 def test_order(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout
+
+
+def test_no_transfer_left_in_flight(program):
+    r = subprocess.run([program, "record_fails"], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout
