@@ -191,6 +191,17 @@ cudaError_t host_copy(void* dst, const void* src, size_t bytes, bool to_device, 
   // the caller's work: the driver's copy, from the calling thread
   bool staged = bytes >= kMinBytes && s != cudaStreamPerThread;
   if (staged) {
+    // a stream in capture: the plain copy and its wait, which ends the capture; transfers queued by the
+    // threads would become part of the caller's graph, with the slots as their memory
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+      cudaGetLastError();
+      staged = false;
+    } else {
+      staged = cs == cudaStreamCaptureStatusNone;
+    }
+  }
+  if (staged) {
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
       cudaGetLastError();

@@ -32,6 +32,7 @@ std::map<Key, Queue> queues;
 std::thread::id caller;
 int staged_copies = 0;     // transfers queued by a thread that is not the caller
 int records = 0, fail_record = -1;
+cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
 
 Queue* queue_of(cudaStream_t s) {
   return &queues[Key(s, s == cudaStreamPerThread ? std::this_thread::get_id() : std::thread::id())];
@@ -93,8 +94,13 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cu
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) {
   std::lock_guard<std::mutex> lk(mu);
+  if (capture != cudaStreamCaptureStatusNone) return cudaErrorStreamCaptureUnsupported;
   Queue* q = queue_of(s);
   run(q, q->ops.size());
+  return cudaSuccess;
+}
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* st) {
+  *st = capture;
   return cudaSuccess;
 }
 }
@@ -153,6 +159,12 @@ int main(int argc, char** argv) {
       CHECK(dev == want);
     }
     CHECK(staged_copies > 0);
+  } else if (!std::strcmp(what, "capture")) {
+    // a stream in capture: no other thread adds to the caller's graph, and the call is refused as a
+    // plain copy with its wait is
+    capture = cudaStreamCaptureStatusActive;
+    CHECK(tg::host_copy(dev.data(), want.data(), n, true, 0, s) == cudaErrorStreamCaptureUnsupported);
+    CHECK(staged_copies == 0);
   } else {
     return 2;
   }

@@ -1,6 +1,6 @@
 """The threaded host copies against a fake CUDA runtime (tests/cpp/hostcopy_fake.cc): streams that run
-nothing until they are waited for, a per-thread stream handle that names another queue in every thread, and an
-event that cannot be recorded."""
+nothing until they are waited for, a per-thread stream handle that names another queue in every thread, an
+event that cannot be recorded, a stream in capture."""
 
 import os
 import shutil
@@ -31,4 +31,9 @@ def test_order(program, scenario):
 
 def test_no_transfer_left_in_flight(program):
     r = subprocess.run([program, "record_fails"], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout
+
+
+def test_stream_in_capture(program):
+    r = subprocess.run([program, "capture"], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout
