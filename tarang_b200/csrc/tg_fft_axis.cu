@@ -4,9 +4,9 @@
 // rows) run k_axis_tma: the block's column tile moves HBM -> shared memory and back as single
 // tiled bulk tensor copies, so the threads spend no instructions on addresses or row maps of
 // global memory.  Power-of-two lengths beyond that run the register-staged k_axis_c2c, every
-// other length the mixed-radix k_axis_mixed.  k_axis_tma and k_axis_c2c compute the same
-// butterflies in the same order (equal results up to how the compiler contracts multiply-adds in
-// each kernel).
+// other length the mixed-radix k_axis_mixed, or the direct sum k_axis_dft where that is faster.
+// k_axis_tma and k_axis_c2c compute the same butterflies in the same order (equal results up to
+// how the compiler contracts multiply-adds in each kernel).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -256,6 +256,31 @@ cudaError_t run_axis_mixed(const AxisLaunch& l, cudaStream_t s) {
   return e;
 }
 
+// The launches of the direct sum (k_axis_dft) among those of no power of two.  Measured in a chain of launches
+// (B200, us, direct / mixed-radix, FP64):
+//  * a prime factor of 11 and more, up to 26, any size: 4 x 4096 columns of 13 6.0 / 8.2, 23 8.7 / 10.9, 26 10.3 / 11.4
+//    (29 12.4 / 12.4, 34 17.1 / 15.6); 4 x 256 columns 2.0 / 2.5, 2.4 / 3.0, 2.5 / 3.0;
+//  * up to 14 where one request has two blocks an SM or less, a chain of latencies: 4 x 256 columns of 6 1.8 / 2.7, 10
+//    1.9 / 3.4, 12 2.0 / 3.7; larger requests go the other way (4 x 2048 columns 3.2 / 3.0, 3.8 / 3.7, 4.0 / 4.0).
+//    From 15 on a lone request gains as well (20 x 24 x 32 MHD FP32-mixed step 82 / 98), but a batch, which takes a lone
+//    request's path, loses more than a tenth (64 requests 844 / 711).
+constexpr int kDftMaxPrime = 26, kDftMax = 14;
+constexpr long long kDftMaxBlocks = 2 * 148;
+bool dft_taken(const AxisLaunch& l) {
+  int m = l.L;
+  for (int q : {2, 3, 5, 7})
+    while (m % q == 0) m /= q;
+  if (m > 1) return l.L <= kDftMaxPrime;
+  const long long blocks = (long long)((l.a.ncols + kDftCols - 1) / kDftCols) * (l.nbatch / l.nreq) * l.nfields;
+  return l.L <= kDftMax && blocks <= kDftMaxBlocks;
+}
+template <typename Ri, typename Ro, typename Rw, int DIR>
+cudaError_t run_axis_dft(const AxisLaunch& l, cudaStream_t s) {
+  const size_t smem = (size_t)l.L * (1 + kDftCols) * sizeof(cx<Rw>);  // 3.7 KB at most
+  dim3 grid((l.a.ncols + kDftCols - 1) / kDftCols, l.nbatch, l.nfields);
+  return launch_pdl(k_axis_dft<Ri, Ro, Rw, DIR>, grid, kDftThreads, smem, s, l.a, l.ps, l.L);
+}
+
 template <typename Ri, typename Ro, typename Rw, int DIR>
 cudaError_t run_axis_dir(const AxisLaunch& l, cudaStream_t s) {
   switch (l.L) {
@@ -270,6 +295,7 @@ cudaError_t run_axis_dir(const AxisLaunch& l, cudaStream_t s) {
     case 512: return run_axis_fast<Ri, Ro, Rw, 32, 16, DIR>(l, s);
     default:
       if (l.L < 1 || l.L > 2048) return cudaErrorInvalidValue;
+      if (dft_taken(l)) return run_axis_dft<Ri, Ro, Rw, DIR>(l, s);
       return run_axis_mixed<Ri, Ro, Rw, DIR>(l, s);
   }
 }

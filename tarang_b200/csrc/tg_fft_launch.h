@@ -13,6 +13,7 @@ struct AxisLaunch {
   int dir = -1;  // -1 forward (e^{-i}), +1 inverse
   int pin = F64, pout = F64, pwork = F64;
   int nbatch = 1, nfields = 1;
+  int nreq = 1;  // requests that share the launch: nbatch / nreq of it are one request's
   AxisArgs a{};
   PtrSet ps{};
 };

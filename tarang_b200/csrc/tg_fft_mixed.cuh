@@ -274,6 +274,56 @@ __global__ void __launch_bounds__(kMixThreads, sizeof(Rw) == 8 ? 4 : 6)
   }
 }
 
+// The direct sum, for short lengths: a thread owns one output of a tile of eight columns.  Bound by latency: two
+// trips to memory and a loop of L terms, in a kernel of few instructions, where the mixed-radix kernel fetches a
+// stage's code per stage and a prime stage, with (r + 1) / 2 outputs a column, leaves most of its block idle.  The
+// times of both stand at the dispatch (dft_taken).
+constexpr int kDftThreads = 256;
+constexpr int kDftCols = 8;
+template <typename Ri, typename Ro, typename Rw, int DIR>
+__global__ void __launch_bounds__(kDftThreads) k_axis_dft(AxisArgs a, PtrSet ps, int L) {
+  constexpr int W = kDftCols;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cx<Rw>* tw = reinterpret_cast<cx<Rw>*>(smem_raw);
+  cx<Rw>* tile = tw + L;  // [L][W]
+  for (int i = threadIdx.x; i < L; i += kDftThreads) {
+    cx<Rw> t = cvt<Rw>(a.tw[i]);
+    if (DIR > 0) t.y = -t.y;
+    tw[i] = t;
+  }
+  pdl_wait();
+  const int f = blockIdx.z;
+  const int comb = a.comb[f];
+  const cx<Ri>* src = reinterpret_cast<const cx<Ri>*>(ps.src[f]) + (long long)blockIdx.y * a.sb;
+  const cx<Ri>* src2 = comb ? reinterpret_cast<const cx<Ri>*>(ps.src2[f]) + (long long)blockIdx.y * a.sb : src;
+  cx<Ro>* dst = reinterpret_cast<cx<Ro>*>(ps.dst[f]) + (long long)blockIdx.y * a.db;
+  const int c0 = blockIdx.x * W;
+  for (int i = threadIdx.x; i < L * W; i += kDftThreads) {
+    const int r = amap_row(a.in, i / W), col = c0 + i % W;
+    cx<Rw> v = mkc<Rw>(0, 0);
+    if (r >= 0 && col < a.ncols) {
+      const long long o = (long long)r * a.sr + col;
+      v = cvt<Rw>(src[o]);
+      if (comb > 0) v = v + cvt<Rw>(src2[o]);
+      else if (comb < 0) v = v - cvt<Rw>(src2[o]);
+    }
+    tile[i] = v;
+  }
+  __syncthreads();
+  const Rw sc = (Rw)a.scale;
+  for (int i = threadIdx.x; i < L * W; i += kDftThreads) {
+    const int k = i / W, w = i % W, r = amap_row(a.out, k), col = c0 + w;
+    if (r < 0 || col >= a.ncols) continue;
+    cx<Rw> acc = mkc<Rw>(0, 0);
+    for (int n = 0, m = 0; n < L; ++n) {
+      acc = acc + tile[n * W + w] * tw[m];
+      m += k;
+      if (m >= L) m -= L;
+    }
+    dst[(long long)r * a.dr + col] = cvt<Ro>(sc * acc);
+  }
+}
+
 // the fewest register stages whose product is the smooth part of L, of those the ones with the
 // smallest largest radix; then the primes of 11 and more.  false: more stages than a plan holds
 inline bool mix_plan(int L, MixPlan& p) {

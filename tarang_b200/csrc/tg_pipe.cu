@@ -67,6 +67,7 @@ int pipe_inverse_xy(tg_ctx* c, int nf, const void* const* in, const void* const*
     l.pout = c->tprec;
     l.pwork = c->tprec;
     l.nbatch = c->nact;
+    l.nreq = c->nact;
     l.nfields = nf;
     l.a.sb = g.S;  // request stride of the batch
     l.a.sr = (long long)g.nky * g.kzp;
@@ -110,6 +111,7 @@ int pipe_inverse_xy(tg_ctx* c, int nf, const void* const* in, const void* const*
     l.dir = +1;
     l.pin = l.pout = l.pwork = c->tprec;
     l.nbatch = c->nact * c->N1;
+    l.nreq = c->nact;
     l.nfields = nf;
     l.a.sb = (long long)g.nky * g.kzp;
     l.a.sr = g.kzp;
@@ -166,6 +168,7 @@ int pipe_products_forward(tg_ctx* c, int nin, const void* const* WY, int nprod, 
     l.dir = -1;
     l.pin = l.pout = l.pwork = c->tprec;
     l.nbatch = c->nact * c->N1;
+    l.nreq = c->nact;
     l.nfields = nprod;
     l.a.sb = (long long)c->N2 * g.kzp;
     l.a.sr = g.kzp;
@@ -216,6 +219,7 @@ int pipe_forward_x(tg_ctx* c, int nprod, void* const* PY, void* const* PX, const
     l.dir = -1;
     l.pin = l.pout = l.pwork = c->tprec;
     l.nbatch = c->nact;
+    l.nreq = c->nact;
     l.nfields = nprod;
     l.a.sb = (long long)c->N1 * g.nky * g.kzp;
     l.a.sr = (long long)g.nky * g.kzp;
