@@ -31,6 +31,7 @@ std::mutex mu;
 std::map<Key, Queue> queues;
 std::thread::id caller;
 int staged_copies = 0;     // transfers queued by a thread that is not the caller
+int allocs = 0;            // of page-locked memory
 int records = 0, fail_record = -1;
 cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
 
@@ -52,6 +53,7 @@ extern "C" {
 int get_nprocs() { return 16; }  // what std::thread::hardware_concurrency reads
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
   *p = std::malloc(n);
+  ++allocs;
   return cudaSuccess;
 }
 cudaError_t cudaFreeHost(void* p) {
@@ -121,6 +123,13 @@ int main(int argc, char** argv) {
   caller = std::this_thread::get_id();
   cudaStream_t s = std::strstr(what, "per_thread") ? cudaStreamPerThread : reinterpret_cast<cudaStream_t>(0x1000);
   tg::host_copy_retain();
+  // the threads come once enough has been copied to pay for them
+  if (std::strcmp(what, "short_use") && std::strcmp(what, "capture")) {
+    const cudaStream_t other = reinterpret_cast<cudaStream_t>(0x2000);
+    for (int i = 0; i < 30; ++i) CHECK(tg::host_copy(dev.data(), host.data(), n, true, 0, other) == cudaSuccess);
+    CHECK(staged_copies > 0);
+    staged_copies = 0;
+  }
 
   if (!std::strcmp(what, "download") || !std::strcmp(what, "download_per_thread")) {
     // work queued before the copy on the caller's stream fills the device buffer
@@ -159,6 +168,20 @@ int main(int argc, char** argv) {
       CHECK(dev == want);
     }
     CHECK(staged_copies > 0);
+  } else if (!std::strcmp(what, "short_use")) {
+    // 13 of the 9 MB copies are 123 MB: owners that come and go with as many never set the threads up
+    for (int round = 0; round < 3; ++round) {
+      for (int i = 0; i < 13; ++i) {
+        CHECK(tg::host_copy(host.data(), want.data(), n, false, 0, s) == cudaSuccess);
+        CHECK(host == want);
+      }
+      CHECK(staged_copies == 0 && allocs == 0);
+      tg::host_copy_release();
+      tg::host_copy_retain();
+    }
+    for (int i = 0; i < 30; ++i) CHECK(tg::host_copy(host.data(), want.data(), n, false, 0, s) == cudaSuccess);
+    CHECK(staged_copies > 0 && allocs == 1);
+    CHECK(host == want);
   } else if (!std::strcmp(what, "capture")) {
     // a stream in capture: no other thread adds to the caller's graph, and the call is refused as a
     // plain copy with its wait is

@@ -1,6 +1,6 @@
 """The threaded host copies against a fake CUDA runtime (tests/cpp/hostcopy_fake.cc): streams that run
 nothing until they are waited for, a per-thread stream handle that names another queue in every thread, an
-event that cannot be recorded, a stream in capture."""
+event that cannot be recorded, a stream in capture, owners that copy too little to pay for the threads."""
 
 import os
 import shutil
@@ -36,4 +36,9 @@ def test_no_transfer_left_in_flight(program):
 
 def test_stream_in_capture(program):
     r = subprocess.run([program, "capture"], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout
+
+
+def test_short_use_sets_up_nothing(program):
+    r = subprocess.run([program, "short_use"], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout
