@@ -124,7 +124,7 @@ int main(int argc, char** argv) {
   cudaStream_t s = std::strstr(what, "per_thread") ? cudaStreamPerThread : reinterpret_cast<cudaStream_t>(0x1000);
   tg::host_copy_retain();
   // the threads come once enough has been copied to pay for them
-  if (std::strcmp(what, "short_use") && std::strcmp(what, "capture")) {
+  if (std::strcmp(what, "short_use")) {
     const cudaStream_t other = reinterpret_cast<cudaStream_t>(0x2000);
     for (int i = 0; i < 30; ++i) CHECK(tg::host_copy(dev.data(), host.data(), n, true, 0, other) == cudaSuccess);
     CHECK(staged_copies > 0);
