@@ -358,10 +358,10 @@ bool r2r_foldable(const AxisLaunch& l, const R2RArgs& r, bool& fwd) {
 }
 
 template <typename Ri, int RT, bool FWD>
-cudaError_t run_r2r_fold_rt(const AxisLaunch& l, const R2RArgs& r, int ntile, int steps, bool vec, cudaStream_t s) {
+cudaError_t run_r2r_fold_rt(const AxisLaunch& l, const R2RArgs& r, int ntile, int steps, cudaStream_t s) {
   const size_t smem = (size_t)kFoldAhead * 2 * kFoldCols * sizeof(cx<Ri>) +
                       (size_t)steps * ((RT + 3) / 4 * 8) * sizeof(float);
-  auto kern = vec ? k_axis_r2r_fold<Ri, RT, FWD, true> : k_axis_r2r_fold<Ri, RT, FWD, false>;
+  auto kern = k_axis_r2r_fold<Ri, RT, FWD>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;
@@ -381,19 +381,18 @@ cudaError_t run_r2r_fold(const AxisLaunch& l, const R2RArgs& r, cudaStream_t s, 
   const int pairs = fwd ? (nout + 1) / 2 : (N + 1) / 2, steps = fwd ? (N + 1) / 2 : (nin + 1) / 2;
   const long long blocks = (long long)((l.a.ncols + kFoldCols - 1) / kFoldCols) * l.nbatch * l.nfields * ((pairs + 21) / 22);
   const int rt = blocks < 2 * 148 ? 11 : 22, ntile = (pairs + rt - 1) / rt;
-  bool vec = ((l.a.ncols | l.a.sr | l.a.dr | l.a.sb | l.a.db) & 1) == 0;
-  for (int f = 0; f < l.nfields; ++f) {
-    const uintptr_t sp = reinterpret_cast<uintptr_t>(l.ps.src[f]), dp = reinterpret_cast<uintptr_t>(l.ps.dst[f]);
-    if (sizeof(Ri) == 8 && (sp & 15)) return cudaSuccess;  // 16-byte copies of complex double columns
-    vec = vec && ((sp | dp) & 15) == 0;
-  }
+  // 16-byte accesses of a thread's two columns: even column counts and strides (whole rows of kzp, a multiple of 8,
+  // on every caller) and aligned buffers
+  if (((l.a.ncols | l.a.sr | l.a.dr | l.a.sb | l.a.db) & 1) != 0) return cudaSuccess;
+  for (int f = 0; f < l.nfields; ++f)
+    if (((reinterpret_cast<uintptr_t>(l.ps.src[f]) | reinterpret_cast<uintptr_t>(l.ps.dst[f])) & 15) != 0) return cudaSuccess;
   if ((long long)l.nfields * ntile > 65535 || (size_t)steps * 48 * sizeof(float) > 96 * 1024) return cudaSuccess;
   *used = true;
   if (rt == 22)
-    return fwd ? run_r2r_fold_rt<Ri, 22, true>(l, r, ntile, steps, vec, s)
-               : run_r2r_fold_rt<Ri, 22, false>(l, r, ntile, steps, vec, s);
-  return fwd ? run_r2r_fold_rt<Ri, 11, true>(l, r, ntile, steps, vec, s)
-             : run_r2r_fold_rt<Ri, 11, false>(l, r, ntile, steps, vec, s);
+    return fwd ? run_r2r_fold_rt<Ri, 22, true>(l, r, ntile, steps, s)
+               : run_r2r_fold_rt<Ri, 22, false>(l, r, ntile, steps, s);
+  return fwd ? run_r2r_fold_rt<Ri, 11, true>(l, r, ntile, steps, s)
+             : run_r2r_fold_rt<Ri, 11, false>(l, r, ntile, steps, s);
 }
 
 // shared memory of k_axis_r2r_dmma: the ring of input stages and the block's coefficients

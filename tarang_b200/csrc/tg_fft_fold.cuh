@@ -33,9 +33,9 @@ constexpr int kFoldThreads = 128;
 constexpr int kFoldCols = 2 * kFoldThreads;  // complex columns of a block, two a thread
 constexpr int kFoldAhead = 8;                // steps in the ring
 
-// VEC: 16-byte accesses of a thread's two columns (even column counts and strides, aligned buffers).
+// Even column counts and strides and 16-byte aligned buffers (run_r2r_fold).
 // grid (column blocks, nbatch, nfields * ntile)
-template <typename Ri, int RT, bool FWD, bool VEC>
+template <typename Ri, int RT, bool FWD>
 __global__ void __launch_bounds__(kFoldThreads, RT <= 11 ? 3 : 2)
     k_axis_r2r_fold(AxisArgs a, PtrSet ps, R2RArgs r, int N, int ntile) {
   pdl_wait();
@@ -54,21 +54,16 @@ __global__ void __launch_bounds__(kFoldThreads, RT <= 11 ? 3 : 2)
   const int steps = FWD ? H : (nin + 1) / 2;
   const int i0 = tile * RT;
   const int col = blockIdx.x * kFoldCols + 2 * threadIdx.x;
-  const bool any = col < a.ncols, both = VEC || col + 1 < a.ncols;
+  const bool any = col < a.ncols;
   const cx<Ri>* src = reinterpret_cast<const cx<Ri>*>(ps.src[f]) + (long long)blockIdx.y * a.sb + col;
   const unsigned ring_s = (unsigned)__cvta_generic_to_shared(ring);
   auto copy = [&](unsigned off, const cx<Ri>* p) {
-    if constexpr (NQ == 1 && VEC) {
+    if constexpr (NQ == 1) {
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring_s + off), "l"(p) : "memory");
     } else {
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        if (c == 1 && !both) continue;
-        if constexpr (NQ == 1)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(ring_s + off + 8 * c), "l"(p + c) : "memory");
-        else
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring_s + off + QB * c), "l"(p + c) : "memory");
-      }
+      for (int c = 0; c < 2; ++c)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring_s + off + QB * c), "l"(p + c) : "memory");
     }
   };
   auto column = [&](const unsigned char* row, int c) {
@@ -154,12 +149,7 @@ __global__ void __launch_bounds__(kFoldThreads, RT <= 11 ? 3 : 2)
   const float sc = (float)a.scale;
   auto store = [&](int row, cx<float> w0, cx<float> w1) {
     cx<float>* p = dst + (long long)row * a.dr;
-    if constexpr (VEC) {
-      *reinterpret_cast<float4*>(p) = make_float4(sc * w0.x, sc * w0.y, sc * w1.x, sc * w1.y);
-    } else {
-      p[0] = sc * w0;
-      if (both) p[1] = sc * w1;
-    }
+    *reinterpret_cast<float4*>(p) = make_float4(sc * w0.x, sc * w0.y, sc * w1.x, sc * w1.y);
   };
 #pragma unroll
   for (int i = 0; i < RT; ++i) {

@@ -251,27 +251,29 @@ cudaError_t run_zprod_m(const ZProdLaunch& l, cudaStream_t s) {
     if constexpr (NIN == 6 && !kTf)
       if (ph == 3) return run_zprod_oct64_any<Ri, Ro, Rw, 3, false>(l, s);
   }
-  // the fourth parked row of the trace-free MHD form does not fit two FP64 blocks of k_z_prod_oct an SM
-  constexpr bool kNoOct = NIN == 6 && kTf && sizeof(Rw) == 8;
-  if (!kNoOct && l.M == 128 && l.a.oct && zpass_oct_enabled() && l.a.nin <= 129 && l.a.nout <= 129) {
-    // the paired output stores need even row strides and 2-entry-aligned product buffers
-    bool aligned = (l.a.ds % 2) == 0;
-    for (int q = 0; q < NPROD && aligned; ++q)
-      aligned = (reinterpret_cast<uintptr_t>(l.ps.dst[q]) % (2 * sizeof(cx<Ro>))) == 0;
-    const int ph = aligned ? oct_phys<NIN, NPROD>(l.pp, tf) : -1;
-    if constexpr (!kNoOct)
+  // the fourth parked row of the trace-free MHD form does not fit two FP64 blocks of k_z_prod_oct an SM:
+  // steps of such rows keep the third square (step_trace_free)
+  constexpr bool kNo128 = NIN == 6 && kTf && sizeof(Rw) == 8;
+  if constexpr (!kNo128) {
+    if (l.M == 128 && l.a.oct && zpass_oct_enabled() && l.a.nin <= 129 && l.a.nout <= 129) {
+      // the paired output stores need even row strides and 2-entry-aligned product buffers
+      bool aligned = (l.a.ds % 2) == 0;
+      for (int q = 0; q < NPROD && aligned; ++q)
+        aligned = (reinterpret_cast<uintptr_t>(l.ps.dst[q]) % (2 * sizeof(cx<Ro>))) == 0;
+      const int ph = aligned ? oct_phys<NIN, NPROD>(l.pp, tf) : -1;
       if (ph == kPh) return run_zprod_oct_any<Ri, Ro, Rw, kPh, kTf>(l, s);
-    if constexpr (NIN == 6 && !kTf)
-      if (ph == 3) return run_zprod_oct_any<Ri, Ro, Rw, 3, false>(l, s);
+      if constexpr (NIN == 6 && !kTf)
+        if (ph == 3) return run_zprod_oct_any<Ri, Ro, Rw, 3, false>(l, s);
+    }
+    if (l.M == 128 && zpass_net_enabled()) return run_zprod_net128<Ri, Ro, Rw, NIN, NPROD>(l, s);
+    if (l.M == 128) return run_zprod_warp<Ri, Ro, Rw, 4, NIN, NPROD>(l, s);
   }
-  if (l.M == 128 && zpass_net_enabled()) return run_zprod_net128<Ri, Ro, Rw, NIN, NPROD>(l, s);
   switch (l.M) {
     case 4: return run_zprod_rows<Rw, 2>(l, s);
     case 8: return run_zprod_rows<Rw, 4>(l, s);
     case 16: return run_zprod_rows<Rw, 8>(l, s);
     case 32: return run_zprod_rows<Rw, 16>(l, s);
     case 64: return run_zprod_warp<Ri, Ro, Rw, 2, NIN, NPROD>(l, s);
-    case 128: return run_zprod_warp<Ri, Ro, Rw, 4, NIN, NPROD>(l, s);
     case 256: return run_zprod_warp<Ri, Ro, Rw, 8, NIN, NPROD>(l, s);
     default: return cudaErrorInvalidValue;
   }

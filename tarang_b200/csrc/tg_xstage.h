@@ -16,7 +16,6 @@ struct XStageLaunch {
   int wait_short = 0;
   const void* src[8] = {};  // y-forward outputs [N1][nky][kzp] of the trace-free products
   void* dst[6] = {};        // x-inverse outputs [N1][nky][kzp]
-  int nprod = 0;
 };
 
 // whether a step on this grid runs its non-final stages through launch_xstage (FOUR, N1 of 32 .. 256)
