@@ -308,12 +308,16 @@ cudaError_t run_xstage_p(const XStageLaunch& l, cudaStream_t s, bool* used) {
 
 }  // namespace
 
-// The lines: a grid whose tiles fit one wave of two blocks an SM is a latency chain, where three launches
-// in one win whatever the kernel's own rate.  A larger grid is taken where the fused kernel, at 20 warps an
-// SM, still beats the three passes at 24 to 48: FP64 fluid with N1 = 256 or 64.  Steps measured (fused /
-// separate, us, the y and z passes one by one): 32^3 FP32 fluid 59.6 / 66.5, MHD 67.8 / 76.0; 64^3 FP64 fluid 94.5 / 102.0, scalar 124 / 135,
-// FP32 MHD 98 / 107; 256 x 64 x 64 FP64 256 / 282; 256^3 FP64 2806 / 3000; 64 x 256 x 256 FP64 806 / 829; and
-// against it 64 x 256 x 256 FP32 500 / 475, MHD 901 / 846, 128^3 FP64 463 / 448, 256^3 FP32 1686 / 1647.
+// The lines: a grid whose tiles fit one wave is a latency chain, where three launches in one win whatever the
+// kernel's own rate.  The line is two blocks an SM; FP32 MHD and scalar blocks have 512 threads and run one an SM,
+// so their line is a second wave, which pays when it is at least half full (MHD and scalar steps, fused / separate,
+// us: 64 x 128 x 64, 249 tiles, 164.9 / 167.5 and 151.8 / 151.5; 64 x 96 x 64, 186 tiles, 176.1 / 168.3 and 165.6 /
+// 162.6; 64 x 82 x 64, 159 tiles, 235.4 / 229.2).  A larger grid is taken where the fused kernel, at 20 warps an
+// SM, still beats the three passes at 24 to 48: FP64 fluid with N1 = 256 or 64.  Steps measured (fused / separate,
+// us, the y and z passes one by one): 32^3 FP32 fluid 59.6 / 66.5, MHD 67.8 / 76.0; 64^3 FP64 fluid 94.5 / 102.0,
+// scalar 124 / 135, FP32 MHD 98 / 107; 256 x 64 x 64 FP64 256 / 282; 256^3 FP64 2806 / 3000; 64 x 256 x 256 FP64
+// 806 / 829; and against it 64 x 256 x 256 FP32 500 / 475, MHD 901 / 846, 128^3 FP64 463 / 448, 256^3 FP32
+// 1686 / 1647.
 // Looks at one request's geometry only, so a batched request takes the path of a lone one.
 bool xstage_fits(const Geo& g, int phys, int prec) {
   if (!axis_tma_enabled() || g.basis != 0 || g.x0 != 0 || phys == PH_RB || g.kzp % 8 != 0) return false;
@@ -321,7 +325,9 @@ bool xstage_fits(const Geo& g, int phys, int prec) {
   const bool have = g.N1 == 32 || g.N1 == 64 || (f64_fluid && (g.N1 == 128 || g.N1 == 256));
   if (!have) return false;
   const long long tiles = (long long)g.nky * g.kzp / (prec == F64 ? XW<double>::v : XW<float>::v);
-  return tiles <= 2 * 148 || (f64_fluid && (g.N1 == 64 || g.N1 == 256));
+  if (f64_fluid && (g.N1 == 64 || g.N1 == 256)) return true;
+  const bool one_a_sm = prec == F32 && phys != PH_FLUID;
+  return tiles <= 2 * 148 && !(one_a_sm && tiles > 148 && tiles < 148 + 74);
 }
 
 cudaError_t launch_xstage(const XStageLaunch& l, cudaStream_t s, bool* used) {
