@@ -139,9 +139,6 @@ int max_radius_inside(const tg_ctx* c) {
 }
 
 // ------------------------------------------------------------------ pipeline
-// X-inverse, Y-inverse, fused z-pass (c2r, products, r2c), Y-forward, X-forward.
-// inputs: compact fields of precision inprec.  MHD: in[0..2] = U, in[3..5] = B, the x-pass
-// forms z+ = U + B (fields 0..2) and z- = U - B (fields 3..5).
 // the products of the trace-free form and their buffers
 struct TraceFree {
   ProdPairs pp;
@@ -164,6 +161,10 @@ struct TraceFree {
   }
 };
 
+// X-inverse, Y-inverse, fused z-pass (c2r, products, r2c), Y-forward, X-forward.
+// inputs: compact fields of precision inprec.  MHD: in[0..2] = U, in[3..5] = B, the x-pass
+// forms z+ = U + B (fields 0..2) and z- = U - B (fields 3..5); have_z: in[] holds z+ and z- already.
+// have_x: WX holds the x-inverse of the inputs (in[] is not read).  leave_x: stop before the x-forward.
 // trace_free: the products without the third square, which is taken from the first two
 // (u1u1 - u3u3, u2u2 - u3u3; z+- alike): five products instead of six, eight instead of nine.  Only for a
 // right-hand side that is projected: the velocity's term changes by a gradient.
@@ -382,7 +383,9 @@ int run_stages(tg_ctx* c, int first, bool ring) {
         TG_CK(launch_xstage(x, c->st, &have_x));
       }
       if (have_x) continue;
-      // refused (a tensor map that the driver does not take): the separate passes
+      // refused (a tensor map that the driver does not take): the separate passes.  What they need is there:
+      // this stage's x-inverse has been used from WX (US may hold the force box alone after a fused stage, but
+      // is read by run_force and, with us_all, by k_rk only), and k_rk writes all of US for the next one.
       const TraceFree t(c);
       rc = pipe_forward_x(c, c->nprod - 1, t.PY, t.PX, t.kinds);
       if (rc) return rc;

@@ -1,7 +1,7 @@
 // Strided-axis c2c pass for lengths that are not powers of two: a mixed-radix Stockham FFT.
 //
 // A block transforms W columns of one batch of one field (a tile [L][W]).  The length is split
-// into register radices (2 .. 12, 16) and, for what is left, prime factors of 11 and more.  Stage
+// into register radices (2 .. 8, 10, 12, 16) and, for what is left, prime factors of 11 and more.  Stage
 // by stage, with s the product of the radices done and n = L / s what remains, n = r m:
 //   y[q + s (r p + k)] = w_n^(p k) sum_j x[q + s (p + m j)] w_r^(j k),  p < m, q < s, k < r,
 // which leaves the result in natural order after the last stage.  A register stage gives a thread

@@ -222,8 +222,8 @@ cudaError_t run_plane_n(const PlaneLaunch& l, cudaStream_t s) {
 }  // namespace
 
 // The lines: a block's time does not fall with the number of planes, the three passes' does.  Steps measured
-// (this form / the three passes, us): planes of 32 x 32 gain from 16 of them (FP32 fluid 55.5 / 63.7, FP64 MHD
-// 69.8 / 76.3).  Larger ones: 64 x 64 FP64 fluid 86 / 78 with 16 or 32 planes, 111 / 112 with 48, 90.6 / 96.3
+// (this form / the three passes, us): planes of 32 x 32 gain whatever their number (FP32 fluid with 4 of them
+// 51.0 / 57.6, with 16 55.5 / 63.7; FP64 MHD with 6 75.9 / 80.0, with 16 69.8 / 76.3).  Larger ones: 64 x 64 FP64 fluid 86 / 78 with 16 or 32 planes, 111 / 112 with 48, 90.6 / 96.3
 // with 64 (two blocks each, to 74), 146 / 148 with 80, 148 / 158 with 96, 128 / 150 with 128, 226 / 258 with 256;
 // FP32 fluid 71 / 68, 96 / 100, 76 / 81, 120 / 119, 123 / 125, 103 / 113, 146 / 179; FP32 MHD 88 / 80, 115 / 117,
 // 98 / 98, 150 / 154, 154 / 162, - , 255 / 292; 64 x 32 FP32 MHD 74 / 84 with 64 planes, 150 / 204 with 256;

@@ -11,11 +11,11 @@
 //
 // Bound: memory, and the serial phases of a block.  Per mode and stage the separate passes moved the
 // products twice (written, read), the stage fields twice, and the rest as here; in FP64 at 256^3 (fluid)
-// 1.18 GB a stage against 0.85.  Tiles
-// of 64-byte rows (4 columns in FP64, 8 in FP32) leave shared memory and registers for 640 threads an SM.  At
-// small grids it is three launches of a latency chain in one.  Measured (B200): 226 us a stage at 256^3 FP64
-// against 87 + 106 + 61; the step's times stand at xstage_fits.  Prefetching the state's rows into L2 while the
-// products transform took 195 us to 174 at 256^3 in FP32.
+// 1.18 GB a stage against 0.85.  Tiles of 64-byte rows (4 columns in FP64, 8 in FP32) leave shared memory
+// and registers for 640 threads an SM.  At small grids it is three launches of a latency chain in one.
+// Measured (B200): 226 us a stage at 256^3 FP64 against 87 + 106 + 61; the steps' times stand at
+// xstage_fits.  Prefetching the state's rows into L2 while the products transform: FP64 fluid 64 x 256 x 256
+// 68.6 us a stage without, 60.6 with it; 256^3 227 and 224.
 #include <algorithm>
 #include <cstring>
 
