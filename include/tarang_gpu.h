@@ -432,10 +432,16 @@ int tg_profile_read(tg_ctx* ctx, tg_kernel_stat* out, int max, int* n);
  * TG_ERR_TIMEOUT.
  *
  * TG_DEBUG_SHORT_TMA_WAIT (value 1 / 0) gives the first wait for a tile no polls at all, so
- * every TMA-staged block reports a timeout; value 0 restores the normal limit.  Changing it
- * drops the context's captured step graph.  For tests of the failure path only.
+ * every TMA-staged block reports a timeout; value 0 restores the normal limit.
+ * TG_DEBUG_SHORT_XSTAGE_WAIT does so for the kernel that joins the x-forward, the stage and the
+ * next x-inverse alone.  TG_DEBUG_REFUSE_XSTAGE lets that kernel be refused, as where the driver
+ * takes no tensor map, at the stages of a mask (bit s: stage s, 1..3 of RK4, 7 of RK2); the
+ * separate passes run instead.  Changing one drops the context's captured step graph.  For tests
+ * of the failure paths only.
  * ---------------------------------------------------------------------------------------- */
 #define TG_DEBUG_SHORT_TMA_WAIT 1
+#define TG_DEBUG_SHORT_XSTAGE_WAIT 2
+#define TG_DEBUG_REFUSE_XSTAGE 3
 int tg_debug_set(tg_ctx* ctx, int what, long long value);
 
 /* ------------------------------------------------------------------------------------------

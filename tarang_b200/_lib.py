@@ -19,6 +19,8 @@ TG_ERR_CUDA = -4
 TG_ERR_UNSUPPORTED = -5
 TG_ERR_TIMEOUT = -6
 TG_DEBUG_SHORT_TMA_WAIT = 1
+TG_DEBUG_SHORT_XSTAGE_WAIT = 2
+TG_DEBUG_REFUSE_XSTAGE = 3
 TG_ERR_STATE = -7
 TG_ERR_BUSY = -8
 

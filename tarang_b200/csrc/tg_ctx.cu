@@ -373,14 +373,14 @@ int run_stages(tg_ctx* c, int first, bool ring) {
       x.us_all = (c->coriolis || c->lm) ? 1 : 0;  // the next stage's force reads the whole field
       x.tw = c->tw[c->N1];
       x.wait_flag = c->wait_status;
-      x.wait_short = c->wait_short;
+      x.wait_short = c->wait_short || c->xstage_wait_short;
       for (int q = 0; q < c->nprod - 1; ++q) x.src[q] = c->PY[q < 2 ? q : q + 1];  // as TraceFree
       for (int i = 0; i < c->nin; ++i) x.dst[i] = c->WX[i];
       {
         const double ns = c->nstate, e = el_compact(c);
         const double tot = (stage >= 2 && stage <= 3 ? 2 : (stage == 1 ? 1 : 0)) * ns * e * 16;
         ProfScope pr(c, "x_stage", (c->nprod - 1 + ns) * el_xstage(c) * c->tsz + ns * e * 16 + tot);
-        TG_CK(launch_xstage(x, c->st, &have_x));
+        if (!(c->xstage_refuse >> stage & 1)) TG_CK(launch_xstage(x, c->st, &have_x));
       }
       if (have_x) continue;
       // refused (a tensor map that the driver does not take): the separate passes.  What they need is there:
@@ -1112,10 +1112,14 @@ int tg_ctx_destroy(tg_ctx* c) {
 
 int tg_debug_set(tg_ctx* c, int what, long long value) {
   if (!c) return TG_ERR_ARG;
-  if (what != TG_DEBUG_SHORT_TMA_WAIT || (value != 0 && value != 1)) return TG_ERR_ARG;
+  int* v = what == TG_DEBUG_SHORT_TMA_WAIT      ? &c->wait_short
+           : what == TG_DEBUG_SHORT_XSTAGE_WAIT ? &c->xstage_wait_short
+           : what == TG_DEBUG_REFUSE_XSTAGE     ? &c->xstage_refuse
+                                                : nullptr;
+  if (!v || value < 0 || value > (what == TG_DEBUG_REFUSE_XSTAGE ? 255 : 1)) return TG_ERR_ARG;
   cudaSetDevice(c->dev);
   TG_SYNC(c, "tg_debug_set");
-  c->wait_short = (int)value;
+  *v = (int)value;
   // the step graph holds the pass arguments it was captured with
   if (c->step_graph) {
     cudaGraphExecDestroy(c->step_graph);

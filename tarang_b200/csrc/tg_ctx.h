@@ -84,6 +84,8 @@ struct tg_ctx {
   int* wait_status = nullptr;
   int* h_wait = nullptr;      // pinned host copy of *wait_status
   int wait_short = 0;         // test hook (tg_debug_set): first TMA wait gets no polls
+  int xstage_wait_short = 0;  // test hook: the same in k_xstage alone
+  int xstage_refuse = 0;      // test hook: stages (bit mask) whose fused launch counts as refused
   int ering_cap = 0;
   double* h_pinned = nullptr;  // small pinned host buffer
   double* diag = nullptr;      // diagnostics scratch (spectra, transfer tables)
