@@ -7,7 +7,7 @@
 namespace tg {
 
 // host <-> device copy of `bytes` behind the work of stream s; on success the copy has ended (host buffer and
-// device buffer may be used).  Page-locked host memory, short copies, the first 128 MB since an owner came, the
+// device buffer may be used).  Page-locked host memory, short copies, the first copies since an owner came, the
 // per-thread default stream and a stream in capture go through cudaMemcpyAsync.
 cudaError_t host_copy(void* dst, const void* src, size_t bytes, bool to_device, int device, cudaStream_t s);
 

@@ -2,6 +2,7 @@
 // nothing until they are waited for.  A stream is a queue of operations; cudaStreamPerThread names another
 // queue in every thread.  Each scenario (argv[1]) exits 0 when the copy did what it has to.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <cstdio>
 #include <cstdlib>
@@ -169,19 +170,25 @@ int main(int argc, char** argv) {
     }
     CHECK(staged_copies > 0);
   } else if (!std::strcmp(what, "short_use")) {
-    // 13 of the 9 MB copies are 123 MB: owners that come and go with as many never set the threads up
+    // a few copies of fields that are there: owners that come and go never set the threads up
     for (int round = 0; round < 3; ++round) {
       for (int i = 0; i < 13; ++i) {
         CHECK(tg::host_copy(host.data(), want.data(), n, false, 0, s) == cudaSuccess);
         CHECK(host == want);
       }
+      for (int i = 0; i < 5; ++i) CHECK(tg::host_copy(dev.data(), want.data(), n, true, 0, s) == cudaSuccess);
       CHECK(staged_copies == 0 && allocs == 0);
       tg::host_copy_release();
       tg::host_copy_retain();
     }
-    for (int i = 0; i < 30; ++i) CHECK(tg::host_copy(host.data(), want.data(), n, false, 0, s) == cudaSuccess);
+    // three downloads into pages that are not there yet do
+    for (int i = 0; i < 3; ++i) {
+      void* f = mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+      CHECK(tg::host_copy(f, want.data(), n, false, 0, s) == cudaSuccess);
+      CHECK(std::memcmp(f, want.data(), n) == 0);
+      munmap(f, n);
+    }
     CHECK(staged_copies > 0 && allocs == 1);
-    CHECK(host == want);
   } else if (!std::strcmp(what, "capture")) {
     // a stream in capture: no other thread adds to the caller's graph, and the call is refused as a
     // plain copy with its wait is

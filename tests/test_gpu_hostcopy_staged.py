@@ -1,5 +1,5 @@
-"""Field copies of a context that has moved enough for the copying threads to have been set up (128 MB): whole and
-ragged counts of their pieces, from one thread and from two, come back from the device bit for bit."""
+"""Field copies of a context that has moved enough for the copying threads to have been set up: whole and ragged
+counts of their pieces, from one thread and from two, come back from the device bit for bit."""
 
 import threading
 
