@@ -358,7 +358,7 @@ int run_stages(tg_ctx* c, int first, bool ring) {
     int rc = run_force(c, in, inprec);
     if (rc) return rc;
     const bool tf = step_trace_free(c);
-    const bool fuse = tf && !stage_is_final(stage) && xstage_fits(c->g, c->phys, c->tprec) && c->slab_W == 0;
+    const bool fuse = tf && !stage_is_final(stage) && xstage_fits(c->g, c->phys, c->tprec, c->nact) && c->slab_W == 0;
     rc = run_pipeline(c, in, inprec, tf, have_x, fuse, have_z);
     if (rc) return rc;
     RKArgs a = rk_args(c, stage);

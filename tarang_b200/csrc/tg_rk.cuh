@@ -16,12 +16,27 @@ __device__ __forceinline__ void stc(void* p, long long i, cx<double> v) {
   reinterpret_cast<cx<R>*>(p)[i] = cvt<R>(v);
 }
 
-__device__ __forceinline__ cx<double> kdot(double kx, double ky, double kz, cx<double> a, cx<double> b, cx<double> c) {
-  return mkc<double>(kx * a.x + ky * b.x + kz * c.x, kx * a.y + ky * b.y + kz * c.y);
+// The algebra below is written with its roundings (a product and its sum fused, or a product alone), so that
+// the compiler has no choice of which products to fuse: the stage gives the same bits in every kernel, and a
+// step may take the fused stage kernel or the separate passes by the size of a batch without changing a result.
+__device__ __forceinline__ cx<double> mulr(double s, cx<double> a) { return mkc<double>(__dmul_rn(s, a.x), __dmul_rn(s, a.y)); }
+__device__ __forceinline__ cx<double> fmar(double s, cx<double> a, cx<double> c) {
+  return mkc<double>(__fma_rn(s, a.x, c.x), __fma_rn(s, a.y, c.y));
 }
+// c + i s a
+__device__ __forceinline__ cx<double> ifmar(double s, cx<double> a, cx<double> c) {
+  return mkc<double>(__fma_rn(-s, a.y, c.x), __fma_rn(s, a.x, c.y));
+}
+// |K|^2 of a mode
+__device__ __forceinline__ double mode_k2(double kx, double ky, double kz) {
+  return __fma_rn(kz, kz, __fma_rn(ky, ky, __dmul_rn(kx, kx)));
+}
+// nu + nu_h K^2 (nu exactly when the hyper term is off)
+__device__ __forceinline__ double mode_nu(double nu, double nuh, double K2) { return nuh != 0.0 ? __fma_rn(nuh, K2, nu) : nu; }
+
 // i (kx a + ky b + kz c)
 __device__ __forceinline__ cx<double> ikdot(double kx, double ky, double kz, cx<double> a, cx<double> b, cx<double> c) {
-  return ione(kdot(kx, ky, kz, a, b, c));
+  return ione(fmar(kz, c, fmar(ky, b, mulr(kx, a))));
 }
 
 // ------------------------------------------------------------------ nonlinear-term assembly
@@ -38,15 +53,16 @@ __device__ __forceinline__ cx<double> ikdot(double kx, double ky, double kz, cx<
 struct XDer {
   double kx;
   int scft;
-  __device__ __forceinline__ cx<double> cos_in(cx<double> p) const {
-    return scft ? mkc<double>(-kx * p.x, -kx * p.y) : ione(kx * p);
+  // c + the derivative of p
+  __device__ __forceinline__ cx<double> cos_in(cx<double> p, cx<double> c) const {
+    return scft ? fmar(-kx, p, c) : ifmar(kx, p, c);
   }
-  __device__ __forceinline__ cx<double> sin_in(cx<double> p) const {
-    return scft ? mkc<double>(kx * p.x, kx * p.y) : ione(kx * p);
+  __device__ __forceinline__ cx<double> sin_in(cx<double> p, cx<double> c) const {
+    return scft ? fmar(kx, p, c) : ifmar(kx, p, c);
   }
 };
 __device__ __forceinline__ cx<double> iky_ikz(double ky, double kz, cx<double> b, cx<double> c) {
-  return ione(mkc<double>(ky * b.x + kz * c.x, ky * b.y + kz * c.y));
+  return ione(fmar(kz, c, mulr(ky, b)));
 }
 
 // the products of one mode; the third is zero in the trace-free form
@@ -62,10 +78,10 @@ __device__ __forceinline__ void assemble(const cx<double> (&p)[9], const XDer& d
   if constexpr (PHYS == PH_FLUID || PHYS == PH_SCALAR || PHYS == PH_RB) {
     // parities of the products (RV_Forward_transform_RSprod Rvf.cc:179-186): u1u1, u2u2, u3u3,
     // u2u3 cos; u1u2, u3u1 sin; and u1 th cos, u2 th, u3 th sin (compute_nlin_SF.cc:80-115)
-    n[0] = dx.cos_in(p[0]) + iky_ikz(ky, kz, p[3], p[5]);
-    n[1] = dx.sin_in(p[3]) + iky_ikz(ky, kz, p[1], p[4]);
-    n[2] = dx.sin_in(p[5]) + iky_ikz(ky, kz, p[4], p[2]);
-    if constexpr (PHYS != PH_FLUID) n[3] = dx.cos_in(p[6]) + iky_ikz(ky, kz, p[7], p[8]);
+    n[0] = dx.cos_in(p[0], iky_ikz(ky, kz, p[3], p[5]));
+    n[1] = dx.sin_in(p[3], iky_ikz(ky, kz, p[1], p[4]));
+    n[2] = dx.sin_in(p[5], iky_ikz(ky, kz, p[4], p[2]));
+    if constexpr (PHYS != PH_FLUID) n[3] = dx.cos_in(p[6], iky_ikz(ky, kz, p[7], p[8]));
   } else {
     const double kx = dx.kx;
     // Zp.nlin (n) and Zm.nlin (nw)
@@ -95,14 +111,11 @@ struct NState {
 // with parity 0; Compute_rhs); other fields rhs = -(nlin - f).
 __device__ __forceinline__ void project_rhs(cx<double>* r, int ns, const XDer& dx, double ky, double kz, double K2) {
   cx<double> p = mkc<double>(0, 0);
-  if (K2 > 0) {
-    const cx<double> div = dx.sin_in(r[0]) + iky_ikz(ky, kz, r[1], r[2]);
-    p = (1.0 / K2) * div;
-  }
-  const cx<double> g0 = dx.cos_in(p), g1 = ione(ky * p), g2 = ione(kz * p);
-  r[0] = mkc<double>(-(r[0].x + g0.x), -(r[0].y + g0.y));
-  r[1] = mkc<double>(-(r[1].x + g1.x), -(r[1].y + g1.y));
-  r[2] = mkc<double>(-(r[2].x + g2.x), -(r[2].y + g2.y));
+  if (K2 > 0) p = mulr(1.0 / K2, dx.sin_in(r[0], iky_ikz(ky, kz, r[1], r[2])));
+  const cx<double> q0 = dx.cos_in(p, r[0]), q1 = ifmar(ky, p, r[1]), q2 = ifmar(kz, p, r[2]);
+  r[0] = mkc<double>(-q0.x, -q0.y);
+  r[1] = mkc<double>(-q1.x, -q1.y);
+  r[2] = mkc<double>(-q2.x, -q2.y);
   for (int c = 3; c < ns; ++c) r[c] = mkc<double>(-r[c].x, -r[c].y);
 }
 
@@ -123,19 +136,19 @@ __device__ __forceinline__ void sub_forces(const RKArgs& a, long long gi, int kx
     cx<double> v[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) v[c] = a.inprec ? ldc<float>(a.IN[c], gi) : ldc<double>(a.IN[c], gi);
-    r[0] = r[0] - (a.om[1] * v[2] - a.om[2] * v[1]);
-    r[1] = r[1] - (a.om[2] * v[0] - a.om[0] * v[2]);
-    r[2] = r[2] - (a.om[0] * v[1] - a.om[1] * v[0]);
+    r[0] = r[0] - fmar(a.om[1], v[2], mulr(-a.om[2], v[1]));
+    r[1] = r[1] - fmar(a.om[2], v[0], mulr(-a.om[0], v[2]));
+    r[2] = r[2] - fmar(a.om[0], v[1], mulr(-a.om[1], v[0]));
   }
   if (a.lm) {
     // Compute_force_Liquid_metal (compute_force_LM.cc:46-70): Force = -(B0 . K)^2/K^2 V
     // (Array_mult_V0_khat_sqr_FOUR four_basic.cc:413-439), then Add_force: nlin -= Force
-    const double bk = a.b0[0] * kx + a.b0[1] * ky + a.b0[2] * kz;
-    const double f = K2 > 0 ? bk * bk / K2 : 0.0;
+    const double bk = __fma_rn(a.b0[0], kx, __fma_rn(a.b0[1], ky, __dmul_rn(a.b0[2], kz)));
+    const double f = K2 > 0 ? __dmul_rn(bk, bk) / K2 : 0.0;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const cx<double> v = a.inprec ? ldc<float>(a.IN[c], gi) : ldc<double>(a.IN[c], gi);
-      r[c] = r[c] + f * v;
+      r[c] = fmar(f, v, r[c]);
     }
   }
   if constexpr (PHYS == PH_RB) {
@@ -143,8 +156,8 @@ __device__ __forceinline__ void sub_forces(const RKArgs& a, long long gi, int kx
     // nlin1 -= fu * theta, T.nlin -= ft * u1
     const cx<double> th = a.inprec ? ldc<float>(a.IN[3], gi) : ldc<double>(a.IN[3], gi);
     const cx<double> u1 = a.inprec ? ldc<float>(a.IN[0], gi) : ldc<double>(a.IN[0], gi);
-    r[0] = r[0] - a.rb_buoy_u * th;
-    r[3] = r[3] - a.rb_buoy_t * u1;
+    r[0] = fmar(-a.rb_buoy_u, th, r[0]);
+    r[3] = fmar(-a.rb_buoy_t, u1, r[3]);
   }
 }
 
@@ -164,14 +177,14 @@ __device__ __forceinline__ void sub_forces(const RKArgs& a, long long gi, int kx
 // that do not end a step (1, 2, 3, 7); eh = E(1/2), e1 = E(1)
 template <int STAGE>
 __device__ __forceinline__ cx<double> stage_field(cx<double> u0, cx<double> rc, double dt, double eh) {
-  if constexpr (STAGE == 1 || STAGE == 7) return eh * (u0 + (0.5 * dt) * rc);
-  else if constexpr (STAGE == 2) return eh * u0 + (0.5 * dt) * rc;
-  else return eh * (eh * u0 + dt * rc);
+  if constexpr (STAGE == 1 || STAGE == 7) return mulr(eh, fmar(0.5 * dt, rc, u0));
+  else if constexpr (STAGE == 2) return fmar(0.5 * dt, rc, mulr(eh, u0));
+  else return mulr(eh, fmar(dt, rc, mulr(eh, u0)));
 }
 template <int STAGE>
 __device__ __forceinline__ cx<double> stage_total(cx<double> tot, cx<double> rc, double dt, double eh, double e1) {
-  if constexpr (STAGE == 1) return (dt / 6.0) * (e1 * rc);
-  else return tot + (dt / 3.0) * (eh * rc);
+  if constexpr (STAGE == 1) return mulr(dt / 6.0, mulr(e1, rc));
+  else return fmar(dt / 3.0, mulr(eh, rc), tot);
 }
 
 }  // namespace tg

@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(TPB, RKOcc<PHYS>::v) k_rk(RKArgs a) {
     }
     const int kxi = geo_kx(g, r1), kyi = geo_ky(g, r2);
     const double kx = kxi * g.kf0, ky = kyi * g.kf1, kz = l3 * g.kf2;
-    const double K2 = kx * kx + ky * ky + kz * kz;
+    const double K2 = mode_k2(kx, ky, kz);
     cx<double> r[NS];
     if constexpr (SRC == 0) {
       const XDer dx{kx, g.basis};
@@ -124,8 +124,7 @@ __global__ void __launch_bounds__(TPB, RKOcc<PHYS>::v) k_rk(RKArgs a) {
 #pragma unroll
     for (int c = 0; c < NS; ++c) {
       if (c == 0 || nus[c] != nus[c - 1] || nuh[c] != nuh[c - 1]) {
-        // nu + nu_h K^2 (nu exactly when the hyper term is off)
-        const double nuk = nuh[c] != 0.0 ? nus[c] + nuh[c] * K2 : nus[c];
+        const double nuk = mode_nu(nus[c], nuh[c], K2);
         eh = exp(-nuk * 0.5 * dt * K2);
         if constexpr (STAGE == 1 || STAGE == 4 || STAGE == 5) e1 = exp(-nuk * dt * K2);
       }
@@ -419,7 +418,7 @@ __global__ void k_pressure(Geo g, PtrArr6 pa, cx<double>* PR) {
     const double K2 = kx * kx + ky * ky + kz * kz;
     // Compute_divergence_nlin (Xderiv of nlin1 with parity 1) then CS_divide_ksqr (A(0,0,0) = 0)
     const XDer dx{kx, g.basis};
-    if (K2 > 0) p = (1.0 / K2) * (dx.sin_in(pa.p[0][idx]) + iky_ikz(ky, kz, pa.p[1][idx], pa.p[2][idx]));
+    if (K2 > 0) p = mulr(1.0 / K2, dx.sin_in(pa.p[0][idx], iky_ikz(ky, kz, pa.p[1][idx], pa.p[2][idx])));
   }
   PR[idx] = p;
 }
@@ -434,10 +433,9 @@ __global__ void k_rhs_from_nlin(Geo g, int ns, PtrArr6 pa, const cx<double>* PR)
   const double kx = geo_kx(g, r1) * g.kf0, ky = geo_ky(g, r2) * g.kf1, kz = l3 * g.kf2;
   const cx<double> p = PR[idx];
   // Add_pressure_gradient (Xderiv of p with parity 0, Yderiv, Zderiv); Compute_rhs: nlin = -nlin
-  const cx<double> g0 = XDer{kx, g.basis}.cos_in(p), g1 = ione(ky * p), g2 = ione(kz * p);
-  pa.p[0][idx] = mkc<double>(0, 0) - (pa.p[0][idx] + g0);
-  pa.p[1][idx] = mkc<double>(0, 0) - (pa.p[1][idx] + g1);
-  pa.p[2][idx] = mkc<double>(0, 0) - (pa.p[2][idx] + g2);
+  pa.p[0][idx] = mkc<double>(0, 0) - XDer{kx, g.basis}.cos_in(p, pa.p[0][idx]);
+  pa.p[1][idx] = mkc<double>(0, 0) - ifmar(ky, p, pa.p[1][idx]);
+  pa.p[2][idx] = mkc<double>(0, 0) - ifmar(kz, p, pa.p[2][idx]);
   for (int c = 3; c < ns; ++c) pa.p[c][idx] = mkc<double>(0, 0) - pa.p[c][idx];
 }
 

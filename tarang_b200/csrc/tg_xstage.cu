@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(XProd<PHYS>::v * XGroup<R, R1>::v, x_occ(XProd
       }
       const int kxi = geo_kx(geo, r1);
       const double kx = kxi * geo.kf0, kz = l3 * geo.kf2;
-      const double K2 = kx * kx + ky * ky + kz * kz;
+      const double K2 = mode_k2(kx, ky, kz);
       cx<double> p[9], r[NS];
       p[2] = mkc<double>(0, 0);
 #pragma unroll
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(XProd<PHYS>::v * XGroup<R, R1>::v, x_occ(XProd
 #pragma unroll
       for (int c = 0; c < NS; ++c) {
         if (c == 0 || nus[c] != nus[c - 1] || nuh[c] != nuh[c - 1]) {
-          const double nuk = nuh[c] != 0.0 ? nus[c] + nuh[c] * K2 : nus[c];
+          const double nuk = mode_nu(nus[c], nuh[c], K2);
           eh = exp(-nuk * 0.5 * dt * K2);
           if constexpr (STAGE == 1) e1 = exp(-nuk * dt * K2);
         }
@@ -308,26 +308,30 @@ cudaError_t run_xstage_p(const XStageLaunch& l, cudaStream_t s, bool* used) {
 
 }  // namespace
 
-// The lines: a grid whose tiles fit one wave is a latency chain, where three launches in one win whatever the
-// kernel's own rate.  The line is two blocks an SM; FP32 MHD and scalar blocks have 512 threads and run one an SM,
-// so their line is a second wave, which pays when it is at least half full (MHD and scalar steps, fused / separate,
-// us: 64 x 128 x 64, 249 tiles, 164.9 / 167.5 and 151.8 / 151.5; 64 x 96 x 64, 186 tiles, 176.1 / 168.3 and 165.6 /
-// 162.6; 64 x 82 x 64, 159 tiles, 235.4 / 229.2).  A larger grid is taken where the fused kernel, at 20 warps an
-// SM, still beats the three passes at 24 to 48: FP64 fluid with N1 = 256 or 64.  Steps measured (fused / separate,
-// us, the y and z passes one by one): 32^3 FP32 fluid 59.6 / 66.5, MHD 67.8 / 76.0; 64^3 FP64 fluid 94.5 / 102.0,
-// scalar 124 / 135, FP32 MHD 98 / 107; 256 x 64 x 64 FP64 256 / 282; 256^3 FP64 2806 / 3000; 64 x 256 x 256 FP64
-// 806 / 829; and against it 64 x 256 x 256 FP32 500 / 475, MHD 901 / 846, 128^3 FP64 463 / 448, 256^3 FP32
-// 1686 / 1647.
-// Looks at one request's geometry only, so a batched request takes the path of a lone one.
-bool xstage_fits(const Geo& g, int phys, int prec) {
+// The lines.  One request: a grid whose tiles fit one wave is a latency chain, where three launches in one win
+// whatever the kernel's own rate: two blocks an SM, or one of the 512 threads of the FP32 MHD and scalar forms (64 x 96
+// x 64, 186 tiles, fused / separate, us a step: 176.1 / 168.3 and 165.6 / 162.6; 64 x 64 x 128, 252 tiles, 149.8 / 142.5
+// and 133.6 / 133.4).  A larger grid is taken where the fused kernel, at 20 warps an SM, still beats the three passes at
+// 24 to 48: FP64 fluid with N1 = 256 or 64.  Steps measured (fused / separate, us, the y and z passes one by one): 32^3
+// FP32 fluid 59.6 / 66.5, MHD 67.8 / 76.0; 64^3 FP64 fluid 94.5 / 102.0, scalar 124 / 135, FP32 MHD 98 / 107;
+// 256 x 64 x 64 FP64 256 / 282; 256^3 FP64 2806 / 3000; 64 x 256 x 256 FP64 806 / 829; and against it 64 x 256 x 256
+// FP32 500 / 475, MHD 901 / 846, 128^3 FP64 463 / 448, 256^3 FP32 1686 / 1647.
+// A batch, where one request is taken: as long as its tiles stay within two waves (one of the 512-thread forms),
+// and at any size for FP64 with N1 = 64.  Steps of 4 and of 16 requests: 32^3 FP64 fluid 98 / 109 and 199 / 188, 64^3
+// FP32 fluid 181 / 186 and 546 / 524, 64^3 FP64 scalar 438 / 448 and 1507 / 1522; 32 x 32 x 128 FP32 MHD 229 / 207 and
+// 657 / 563, scalar 202 / 177 and 569 / 472, FP64 MHD 281 / 277 and 884 / 817.
+// Both ways give the same bits (tg_rk.cuh), so a result does not depend on the batch.
+bool xstage_fits(const Geo& g, int phys, int prec, int nact) {
   if (!axis_tma_enabled() || g.basis != 0 || g.x0 != 0 || phys == PH_RB || g.kzp % 8 != 0) return false;
-  const bool f64_fluid = prec == F64 && phys == PH_FLUID;
-  const bool have = g.N1 == 32 || g.N1 == 64 || (f64_fluid && (g.N1 == 128 || g.N1 == 256));
+  const bool f64 = prec == F64, fluid = phys == PH_FLUID;
+  const bool have = g.N1 == 32 || g.N1 == 64 || (f64 && fluid && (g.N1 == 128 || g.N1 == 256));
   if (!have) return false;
-  const long long tiles = (long long)g.nky * g.kzp / (prec == F64 ? XW<double>::v : XW<float>::v);
-  if (f64_fluid && (g.N1 == 64 || g.N1 == 256)) return true;
-  const bool one_a_sm = prec == F32 && phys != PH_FLUID;
-  return tiles <= 2 * 148 && !(one_a_sm && tiles > 148 && tiles < 148 + 74);
+  const long long tiles = (long long)g.nky * g.kzp / (f64 ? XW<double>::v : XW<float>::v);
+  if (f64 && fluid && (g.N1 == 64 || g.N1 == 256)) return true;
+  const bool wide = !f64 && !fluid;  // 512 threads
+  if (tiles > (wide ? 148 : 2 * 148)) return false;
+  if (nact <= 1 || (f64 && g.N1 == 64)) return true;
+  return tiles * nact <= (wide ? 148 : (f64 && fluid ? 2 * 4 * 148 : 2 * 2 * 148));
 }
 
 cudaError_t launch_xstage(const XStageLaunch& l, cudaStream_t s, bool* used) {

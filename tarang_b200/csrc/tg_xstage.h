@@ -18,8 +18,9 @@ struct XStageLaunch {
   void* dst[6] = {};        // x-inverse outputs [N1][nky][kzp]
 };
 
-// whether a step on this grid runs its non-final stages through launch_xstage (FOUR, N1 of 32 .. 256)
-bool xstage_fits(const Geo& g, int phys, int prec);
+// whether a step of nact requests on this grid runs its non-final stages through launch_xstage (FOUR, N1 of
+// 32 .. 256)
+bool xstage_fits(const Geo& g, int phys, int prec, int nact);
 cudaError_t launch_xstage(const XStageLaunch& l, cudaStream_t s, bool* used);
 
 }  // namespace tg

@@ -1,6 +1,6 @@
-"""Steps through k_xstage with every mode stored, box factors other than one and hyper-dissipation, and FP32
-MHD and scalar grids on both sides of its lines (one wave of tiles, a second wave less and more than half full),
-two steps against the oracle: 1e-12 (FP64) and 1e-6 (FP32-mixed) relative L2."""
+"""Steps through k_xstage with every mode stored, box factors other than one and hyper-dissipation, and FP32 MHD and
+scalar grids on both sides of its line (one wave of tiles), against the oracle: 1e-12 (FP64) and 1e-6 (FP32-mixed)
+relative L2."""
 
 import numpy as np
 import pytest
@@ -53,8 +53,8 @@ def test_options(N1, physics, precision, option):
     compare((N1, 10, 16), physics, precision, **option)
 
 
-# tiles of eight columns: 147, 222 and 294 (fused), 150, 219 and 297 (the separate passes)
-@pytest.mark.parametrize("N2", [76, 78, 112, 114, 150, 152])
+# tiles of eight columns: 147 (fused), 150 and 297 (the separate passes)
+@pytest.mark.parametrize("N2", [76, 78, 152])
 @pytest.mark.parametrize("physics", ["MHD", "SCALAR"])
 def test_lines(N2, physics):
     compare((32, N2, 64), physics, "FP32", n=1)
