@@ -9,8 +9,10 @@
 // are broadcast from shared memory; the inputs are copied by cp.async into the thread's own
 // shared-memory ring, kFoldAhead - 1 steps ahead (two warps a scheduler at these registers do not
 // hide a load), so a block has no barrier in its loop.  re and im are multiplied by one packed
-// instruction.  Bound: the FP32 pipe and shared memory into the registers (128 bytes a cycle and SM, a
-// broadcast counts for every lane: 56 cycles a step and warp against 44 of the pipe at RT = 22).
+// instruction.  The limits are the FP32 pipe and shared memory into the registers (128 bytes a cycle and SM,
+// a broadcast counts for every lane: 56 cycles a step and warp against 44 of the pipe at RT = 22); what
+// bounds a launch is latency at those few warps: issue slots 41 % used at 129 x 256 x 256, 34 % at
+// 65 x 128 x 128 forward, 17 % inverse (ncu).
 // Measured (B200, CUDA events around a launch; in brackets the 3xTF32 tensor-core form): 129 x 256 x 256
 // forward of nine fields 115 us [134], 65 x 128 x 128 16.6 [26.1], inverse of four 17.1 [19.4];
 // 33 x 256 x 256 24.8 [47.7] and 19.5 [21.2].  Row groups of one block sharing one staged copy of the

@@ -9,11 +9,13 @@
 // the kept rows back, the stages between move through two shared-memory tiles.
 //
 // What bounds it: a pass moves each value once from and to HBM and once through shared memory per
-// stage boundary, L (r1 + r2 + ..) / 2 operations a column instead of the L^2 of a direct sum, so
-// a two-stage length (96 = 12 x 8) is memory- or latency-bound like the power-of-two passes.  The
-// direct sum that this replaces was bound by shared-memory reads (two per multiply-add).  Measured
-// (B200, passive scalar 96 x 80 x 64 FP64): y-forward of nine fields 26.9 us a launch, was 74.3;
-// x-forward 18.8, was 58.1; y-inverse of four 17.4, was 55.5; a step 0.38 ms, was 1.00.
+// stage boundary, L (r1 + r2 + ..) / 2 operations a column instead of the L^2 of a direct sum.  No unit
+// is near its limit (ncu, 192 x 160 x 128 FP64: HBM 14 to 30 %, FP64 pipe 13 to 16 %): at 24 % of the
+// warps (127 registers) the stages' barriers, fixed latencies and loads are not hidden, and the stage
+// switch has its code fetched anew by short launches.  The direct sum that this replaces was bound by
+// shared-memory reads (two per multiply-add).  Measured (B200, passive scalar 96 x 80 x 64 FP64):
+// y-forward of nine fields 26.9 us a launch, was 74.3; x-forward 18.8, was 58.1; y-inverse of four 17.4,
+// was 55.5; a step 0.34 ms, was 0.98.
 // A prime stage is a direct sum over its r inputs from shared memory, outputs k and r - k
 // together: with A = x_j + x_(r-j), B = x_j - x_(r-j) they share every load and product.
 #pragma once
