@@ -112,10 +112,9 @@ struct NState {
 __device__ __forceinline__ void project_rhs(cx<double>* r, int ns, const XDer& dx, double ky, double kz, double K2) {
   cx<double> p = mkc<double>(0, 0);
   if (K2 > 0) p = mulr(1.0 / K2, dx.sin_in(r[0], iky_ikz(ky, kz, r[1], r[2])));
-  const cx<double> q0 = dx.cos_in(p, r[0]), q1 = ifmar(ky, p, r[1]), q2 = ifmar(kz, p, r[2]);
-  r[0] = mkc<double>(-q0.x, -q0.y);
-  r[1] = mkc<double>(-q1.x, -q1.y);
-  r[2] = mkc<double>(-q2.x, -q2.y);
+  r[0] = dx.cos_in(mkc<double>(-p.x, -p.y), mkc<double>(-r[0].x, -r[0].y));
+  r[1] = ifmar(-ky, p, mkc<double>(-r[1].x, -r[1].y));
+  r[2] = ifmar(-kz, p, mkc<double>(-r[2].x, -r[2].y));
   for (int c = 3; c < ns; ++c) r[c] = mkc<double>(-r[c].x, -r[c].y);
 }
 
